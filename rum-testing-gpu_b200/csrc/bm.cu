@@ -25,6 +25,7 @@
 
 #include "bfly.cuh"
 #include "xform.cuh"
+#include "dr.cuh"
 #include "prox.cuh"
 #include "bm.cuh"
 #include "ctx.cuh"
@@ -566,6 +567,7 @@ struct BmCoef {
     int lo_bits = 12;           // transform window split (tuned)
     int prox_form = PROX_TILE;  // prox kernel form (tuned)
     int fuse = 1;               // two windows: P4 carries the next A' (three passes an iteration; tuned)
+    bool dr = false;            // the two-kernel iteration (dr.cuh)
 };
 
 static BmCoef make_coef(int n, double beta, double alpha, double p) {
@@ -739,10 +741,59 @@ static void enqueue_iteration_ptrs(const IterPtrs<T> &I, const BmCoef &C, int n,
     prof_end(st);
 }
 
+// The two-kernel iteration (dr.cuh) on the same buffers: c and d in x and Ax, the streams in t1 and
+// t2, the thresholds in z (2^n of its n 2^(n-1) values); x2 receives u and s receives t at the end of
+// every sequence, which is when a check or dr_end reads them. y is free in between.
+static DrArgs dr_args(const IterPtrs<double> &I, const BmCoef &C, int n) {
+    DrArgs P{};
+    P.n = n;
+    P.Nloc = 1LL << (n - 1);
+    P.c = I.x; P.d = I.Ax; P.a = I.t1; P.e = I.t2; P.tau = I.z;
+    P.u_out = I.x2; P.t_out = I.s;
+    P.xhat = I.xhat;
+    P.menu_obs = I.menu_obs;
+    P.diag = I.diag + 32;
+    P.kQ = Co<double>{C.Qu[0], C.Qu[1], C.Qu[2], C.Qu[3]};
+    P.kAQ = Co<double>{C.AQu[0], C.AQu[1], C.AQu[2], C.AQu[3]};
+    P.kA = Co<double>{1.0, -1.0, 0.0, C.p};
+    P.kAp = Co<double>{1.0, 0.0, -1.0, C.p};
+    P.alpha = C.alpha; P.b = C.b2;
+    P.inv_c0 = 1.0 / C.b2; P.inv_c1 = 1.0 / (C.b2 + 2.0);
+    P.bstride = P.tstride = I.bstride;
+    P.active = I.active;
+    return P;
+}
+
 // `count` iterations as one sequence (see enqueue_iteration_ptrs) for every slot of I.
 template <class T>
 static void enqueue_iterations_ptrs(const IterPtrs<T> &I, const BmCoef &C, int n, cudaStream_t st, int count) {
+    if constexpr (sizeof(T) == 8) {
+        if (C.dr) {
+            const DrArgs P = dr_args(I, C, n);
+            for (int i = 0; i < count; ++i) dr_iteration(P, I.slots, i + 1 == count, st);
+            return;
+        }
+    }
     for (int i = 0; i < count; ++i) enqueue_iteration_ptrs<T>(I, C, n, st, i, count);
+}
+
+// Around a run of sequences: from the slabs x2, s, y, z (slot `slot` of I, or the only one) into the
+// two-kernel iteration's state, and back. Nothing to do for the other sequences.
+template <class T>
+static void enqueue_begin(const IterPtrs<T> &I, const BmCoef &C, int n, cudaStream_t st, int slot = 0) {
+    if constexpr (sizeof(T) == 8) {
+        if (!C.dr) return;
+        DrArgs P = dr_args(I, C, n);
+        const ll o = (ll)slot * I.bstride;
+        P.c += o; P.d += o; P.a += o; P.e += o; P.tau += o;
+        dr_begin(P, 1, I.x2 + o, I.s + o, I.y + o, I.z + o, st);
+    }
+}
+template <class T>
+static void enqueue_end(const IterPtrs<T> &I, const BmCoef &C, int n, cudaStream_t st) {
+    if constexpr (sizeof(T) == 8) {
+        if (C.dr) dr_end(dr_args(I, C, n), I.x2, I.s, I.y, I.z, st);
+    }
 }
 
 template <class T>
@@ -767,6 +818,10 @@ static void enqueue_iteration(BmWork<T> &W, const BmCoef &C, int n, cudaStream_t
 
 template <class T>
 static void enqueue_iterations(BmWork<T> &W, const BmCoef &C, int n, cudaStream_t st, int count) {
+    if (C.dr) {
+        enqueue_iterations_ptrs<T>(iter_ptrs<T>(W), C, n, st, count);
+        return;
+    }
     for (int i = 0; i < count; ++i) enqueue_iteration<T>(W, C, n, st, i, count);
 }
 
@@ -798,6 +853,12 @@ static int forced_knob(const char *name, int count) {
     int v = atoi(e);
     return (v >= 0 && v < count) ? v : -1;
 }
+// The two-kernel iteration's range: float64 states of n >= DR_MIN_N, unless a knob asks for a form of
+// the other sequences. (A float32 state's bracket follows its rounding, so its arithmetic stays.)
+template <class T>
+static bool takes_dr(int n) {
+    return sizeof(T) == 8 && n >= DR_MIN_N && forced_knob("RUMB_PROX_FORM", PROX_FORMS) < 0 && forced_knob("RUMB_FUSE", 2) < 0;
+}
 static void apply_forced(BmCoef &C) {
     int f = forced_knob("RUMB_PROX_FORM", PROX_FORMS);
     if (f >= 0) C.prox_form = f;
@@ -807,6 +868,8 @@ static void apply_forced(BmCoef &C) {
 
 template <class T>
 static void tune_iteration(Ctx &c, BmWork<T> &W, BmCoef &C, int n, cudaStream_t st) {
+    C.dr = takes_dr<T>(n);
+    if (C.dr) return;                                        // nothing to tune
     auto key = std::make_pair(n, (int)sizeof(T));
     auto it = c.tuned.find(key);
     if (it == c.tuned.end()) {
@@ -869,6 +932,7 @@ static void tune_iteration(Ctx &c, BmWork<T> &W, BmCoef &C, int n, cudaStream_t 
 // The tuned schedule of (n, dtype) when it is known, else the defaults.
 template <class T>
 static void tuned_or_default(Ctx &c, BmCoef &C, int n) {
+    C.dr = takes_dr<T>(n);
     auto it = c.tuned.find(std::make_pair(n, (int)sizeof(T)));
     if (it != c.tuned.end()) {
         C.lo_bits = it->second[0];
@@ -1313,6 +1377,7 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     } else {
         if (warm) copy_state_in<double>(*W64, *warm, m2, st);
         else enqueue_cold_start<double>(*W64, C, n, st);
+        enqueue_begin<double>(iter_ptrs<double>(*W64), C, n, st);
     }
     set_doubles_kernel<<<1, 32, 0, st>>>(CW.res.as<double>(), R_SLOTS, 0.0);
     RUMB_LAUNCH("set_doubles");
@@ -1331,6 +1396,7 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
         bool done = run_leg<float>(c, CW, *W32, C, *pr, *par, L, t0, stall_exit, trace, user);
         if (!done && par->dtype == RUMB_MIXED) {
             promote_state(*W32, *W64, m2, st);
+            enqueue_begin<double>(iter_ptrs<double>(*W64), C64, n, st);
             final_dtype64 = true;
             run_leg<double>(c, CW, *W64, C64, *pr, *par, L, t0, false, trace, user);
         } else if (!done) {
@@ -1343,6 +1409,7 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     if (p_fit && std::isfinite(L.ub))
         RUMB_CUDA(cudaMemcpyAsync(p_fit, CW.pfit_best.ptr, (size_t)pr->mp * 8, cudaMemcpyDeviceToHost, st));
     if (keep) {
+        if (final_dtype64) enqueue_end<double>(iter_ptrs<double>(*W64), C64, n, st);
         *keep = final_dtype64 ? copy_state_out<double>(*W64, n, c.device, st)
                               : copy_state_out<float>(*W32, n, c.device, st);
     }
@@ -1399,7 +1466,11 @@ int bm_iterate(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, voi
             RUMB_CUDA(cudaMemcpyAsync(W.y.ptr, y, sb, cudaMemcpyHostToDevice, st));
             RUMB_CUDA(cudaMemcpyAsync(W.z.ptr, z, sb, cudaMemcpyHostToDevice, st));
         }
-        enqueue_iterations<T>(W, C, n, st, iters);
+        if (iters > 0) {
+            enqueue_begin<T>(iter_ptrs<T>(W), C, n, st);
+            enqueue_iterations<T>(W, C, n, st, iters);
+            enqueue_end<T>(iter_ptrs<T>(W), C, n, st);
+        }
         RUMB_CUDA(cudaMemcpyAsync(x2, W.x2.ptr, sb, cudaMemcpyDeviceToHost, st));
         RUMB_CUDA(cudaMemcpyAsync(s, W.s.ptr, sb, cudaMemcpyDeviceToHost, st));
         RUMB_CUDA(cudaMemcpyAsync(y, W.y.ptr, sb, cudaMemcpyDeviceToHost, st));
@@ -1446,6 +1517,7 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
         enqueue_cold_start<T>(W, C, n, st);
         tune_iteration<T>(c, W, C, n, st);
         enqueue_cold_start<T>(W, C, n, st);
+        enqueue_begin<T>(iter_ptrs<T>(W), C, n, st);
         enqueue_iterations<T>(W, C, n, st, std::max(warmup, 3));      // warm-up
         RUMB_CUDA(cudaStreamSynchronize(st));
         // one check first, so that its cached tables exist before the capture (no allocation inside)
@@ -1716,6 +1788,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
             copy_double_kernel<<<1, 32, 0, st>>>(rk + R_LB_SEED, rk + R_LB_NOW);
             RUMB_LAUNCH("copy_double_kernel");
         }
+        enqueue_begin<T>(I, C, n, st, k);
     };
     for (int k = 0; k < K; ++k) admit(k);
     RUMB_CUDA(cudaMemcpyAsync(W.active.ptr, act.data(), (size_t)K * 4, cudaMemcpyHostToDevice, st));
