@@ -26,6 +26,7 @@
 #include "bfly.cuh"
 #include "xform.cuh"
 #include "dr.cuh"
+#include "cert.cuh"
 #include "prox.cuh"
 #include "bm.cuh"
 #include "ctx.cuh"
@@ -211,135 +212,6 @@ __global__ void obs_setup_kernel(const uint32_t *menu, const int32_t *alt, const
     atomicOr(&obsbits[pos >> 5], 1u << (pos & 31));
 }
 
-// ================================================================= float64 certificate
-// The push works on q = Mobius(x) and recomputes the clipped weights w = max(q, 0) + eps where
-// they are read, instead of storing a w slab.
-__device__ __forceinline__ double wclip(double q, double eps) { return (q > 0.0 ? q : 0.0) + eps; }
-
-__global__ void outw_kernel(const double *q, double *outw, int n, ll Nloc, double eps) {
-    ll D = blockIdx.x * (ll)blockDim.x + threadIdx.x;
-    ll N = 1LL << n;
-    if (D >= N) return;
-    double s = 0.0;
-    for (int x = 0; x < n; ++x) {
-        ll bit = 1LL << x;
-        if (!(D & bit)) s += wclip(q[(ll)x * Nloc + (ll)compress_bit((ull)D, x)], eps);
-    }
-    outw[D] = s;
-}
-
-__global__ void mass_layer_kernel(const double *q, const double *outw, double *mass, const int *nodes, ll ns,
-                                  int n, ll Nloc, double eps) {
-    ll i = blockIdx.x * (ll)blockDim.x + threadIdx.x;
-    if (i >= ns) return;
-    ll C = nodes[i];
-    double s = 0.0;
-    for (int x = 0; x < n; ++x) {
-        ll bit = 1LL << x;
-        if (C & bit) {
-            ll P = C ^ bit;
-            double ow = outw[P];
-            if (ow > 0.0) s += mass[P] * wclip(q[(ll)x * Nloc + (ll)compress_bit((ull)P, x)], eps) / ow;
-        }
-    }
-    mass[C] = s;
-}
-
-__global__ void extract_kernel(const double *q, const double *outw, const double *mass, double *rf, int n,
-                               ll Nloc, double eps) {
-    ll a = blockIdx.x * (ll)blockDim.x + threadIdx.x;
-    ll m2 = (ll)n * Nloc;
-    if (a >= m2) return;
-    ll x = a / Nloc, rest = a - x * Nloc;
-    ll T = (ll)expand_bit((ull)rest, (int)x);
-    double ow = outw[T];
-    rf[a] = (ow > 0.0) ? mass[T] * wclip(q[a], eps) / ow : 0.0;
-}
-
-__global__ void lpath_layer_kernel(const double *R, double *dp, const int *nodes, ll ns, int n, ll Nloc) {
-    ll i = blockIdx.x * (ll)blockDim.x + threadIdx.x;
-    if (i >= ns) return;
-    ll C = nodes[i];
-    double best = -1e300;
-    for (int x = 0; x < n; ++x) {
-        ll bit = 1LL << x;
-        if (C & bit) {
-            ll P = C ^ bit;
-            double v = dp[P] + R[(ll)x * Nloc + (ll)compress_bit((ull)P, x)];
-            if (v > best) best = v;
-        }
-    }
-    dp[C] = best;
-}
-
-constexpr int RED_THREADS = 1024;
-
-// Deterministic single-block sum of the per-thread partials (fixed order for a fixed size).
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x < 32) {
-        r = (l < (int)(blockDim.x >> 5)) ? sh[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    }
-    return r;  // valid in thread 0
-}
-
-// Result slots of one check (device doubles)
-enum { R_PHI2 = 0, R_RY = 1, R_UB_NOW = 2, R_UB_BEST = 3, R_LB_NOW = 4, R_LB_SEED = 5, R_SLOTS = 8 };
-
-// phi^2 = sum (p - x2[obs])^2 and sum (p - y) y at the iterate; LB scatter g[obs] = r if g
-template <class T>
-__global__ void obs_stats_kernel(const T *x2, const ll *obs, const double *p, ll mp, double *g, double *res,
-                                 const double *yv = nullptr) {
-    __shared__ double sh[32];
-    double f = 0.0, ry = 0.0;
-    for (ll j = threadIdx.x; j < mp; j += blockDim.x) {
-        double y = yv ? yv[j] : (double)x2[obs[j]];     // yv: the observed values given directly
-        double r = p[j] - y;
-        f += r * r;
-        ry += r * y;
-        if (g) g[obs[j]] = r;
-    }
-    double F = block_sum(f, sh);
-    double RY = block_sum(ry, sh);
-    if (threadIdx.x == 0) { res[R_PHI2] = F; res[R_RY] = RY; }
-}
-
-__global__ void ub_eval_kernel(const double *xub, const ll *obs, const double *p, ll mp, double *pfit_cur,
-                               double *res) {
-    __shared__ double sh[32];
-    double f = 0.0;
-    for (ll j = threadIdx.x; j < mp; j += blockDim.x) {
-        double v = xub[obs[j]];
-        pfit_cur[j] = v;
-        double d = v - p[j];
-        f += d * d;
-    }
-    double F = block_sum(f, sh);
-    if (threadIdx.x == 0) res[R_UB_NOW] = sqrt(F);
-}
-
-__global__ void ub_commit_kernel(const double *pfit_cur, double *pfit_best, ll mp, const double *res) {
-    ll j = blockIdx.x * (ll)blockDim.x + threadIdx.x;
-    if (j >= mp) return;
-    if (res[R_UB_NOW] < res[R_UB_BEST]) pfit_best[j] = pfit_cur[j];
-}
-
-__global__ void ub_best_kernel(double *res) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && res[R_UB_NOW] < res[R_UB_BEST]) res[R_UB_BEST] = res[R_UB_NOW];
-}
-
-__global__ void lb_final_kernel(const double *dp, ll N, double *res) {
-    double rc = dp[N - 1] - res[R_RY];
-    double v = res[R_PHI2] - 2.0 * rc;
-    res[R_LB_NOW] = sqrt(v > 0.0 ? v : 0.0);
-}
-
 __global__ void set_doubles_kernel(double *p, int count, double v) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count) p[i] = v;
@@ -391,8 +263,9 @@ const int *Ctx::layer_table(int n, std::vector<ll> &bounds) {
 // Generic full transform in -> out (K_PLAIN passes; the certificate's Mobius, zeta and
 // subset-sum butterflies). in may be float32 while out is float64 (the first pass converts).
 template <class T, class TI>
-static void xf_transform(int n, const TI *in, T *out, Co<T> k, cudaStream_t st) {
-    if (n - 1 < 5) {
+static void xf_transform(int n, const TI *in, T *out, Co<T> k, cudaStream_t st, int slots = 1,
+                         const int *active = nullptr) {
+    if (n - 1 < 5) {                                  // one slot at a time (no batch is this small)
         bf_transform<T, TI>(n, in, out, k.a, k.b, k.c, k.d, st);
         return;
     }
@@ -402,38 +275,51 @@ static void xf_transform(int n, const TI *in, T *out, Co<T> k, cudaStream_t st) 
         if (i == 0) {
             XfArgs<T, TI> A{};
             A.in = in; A.out = out; A.k1 = k; A.Nloc = Nloc; A.s0 = plan[i].s0; A.B = plan[i].B;
-            xf_launch<T, TI, K_PLAIN>(A, plan[i], n, st);
+            A.bstride = (ll)n * Nloc; A.active = active;
+            xf_launch<T, TI, K_PLAIN>(A, plan[i], n, st, slots);
         } else {
             XfArgs<T, T> A{};
             A.in = out; A.out = out; A.k1 = k; A.Nloc = Nloc; A.s0 = plan[i].s0; A.B = plan[i].B;
-            xf_launch<T, T, K_PLAIN>(A, plan[i], n, st);
+            A.bstride = (ll)n * Nloc; A.active = active;
+            xf_launch<T, T, K_PLAIN>(A, plan[i], n, st, slots);
         }
     }
 }
 
 // ----------------------------------------------------------------- certificate workspace
+// Slabs and node arrays for `slots` iterates checked together (1, or a batch's share), the rows' and
+// results' arrays of a single solve.
 struct CertWork : public BmWorkBase {
     DevBuf qa, qb;            // float64 slabs
     DevBuf outw, mass, dp;    // float64 node arrays
     DevBuf obs, p;            // observed positions and p (mp)
     DevBuf pfit_cur, pfit_best;
     DevBuf res;               // R_SLOTS doubles
+    DevBuf part, count;       // partial sums and finished CTAs
     ll mp = 0;
     int n = 0;
-    void ensure(int n_, ll mp_) {
+    static size_t slot_bytes(int n, ll mp) {
+        return 2 * 8 * ((size_t)n << (n - 1)) + 3 * ((size_t)8 << n) + 8 * (size_t)mp + CERT_PART * 8 + 8;
+    }
+    void ensure(int n_, ll mp_, int slots = 1) {
         n = n_;
         mp = mp_;
-        ll m2 = (ll)n << (n - 1), N = 1LL << n;
-        qa.ensure((size_t)m2 * 8);
-        qb.ensure((size_t)m2 * 8);
-        outw.ensure((size_t)N * 8);
-        mass.ensure((size_t)N * 8);
-        dp.ensure((size_t)N * 8);
+        const size_t m2 = (size_t)n << (n - 1), N = (size_t)1 << n, K = (size_t)slots;
+        qa.ensure(K * m2 * 8);
+        qb.ensure(K * m2 * 8);
+        outw.ensure(K * N * 8);
+        mass.ensure(K * N * 8);
+        dp.ensure(K * N * 8);
         obs.ensure((size_t)mp * 8);
         p.ensure((size_t)mp * 8);
-        pfit_cur.ensure((size_t)mp * 8);
+        pfit_cur.ensure(K * (size_t)mp * 8);
         pfit_best.ensure((size_t)mp * 8);
         res.ensure(R_SLOTS * 8);
+        part.ensure(K * CERT_PART * 8);
+        if (count.bytes < K * 8) {
+            count.ensure(K * 8);
+            RUMB_CUDA(cudaMemset(count.ptr, 0, K * 8));
+        }
     }
 };
 
@@ -442,71 +328,81 @@ static CertWork &cert_work(Ctx &c) {
     return *static_cast<CertWork *>(c.cert.get());
 }
 
-// UB part of a check: x2 (dtype T) -> q = Mobius -> push -> zeta -> ub_now, pfit; running best.
+// One check's inputs. A single solve: the workspace's rows, results and best point, one slot. A batch: its
+// slots' own, with flags.
 template <class T>
-static void enqueue_push(Ctx &c, CertWork &W, int n, const T *x2, cudaStream_t st, const double *p_ovr = nullptr,
-                         double *res_ovr = nullptr, double *pfit_ovr = nullptr) {
-    const double *pp = p_ovr ? p_ovr : W.p.as<double>();
-    double *rr = res_ovr ? res_ovr : W.res.as<double>();
-    // the best point's observed values: the workspace's own, a batched draw's own row, or none
-    double *pfit_best = res_ovr == nullptr ? W.pfit_best.as<double>() : pfit_ovr;
-    ll Nloc = 1LL << (n - 1), m2 = (ll)n * Nloc, N = 1LL << n;
-    const double eps = 1e-12;
-    double *qa = W.qa.as<double>(), *qb = W.qb.as<double>();
-    xf_transform<double, T>(n, x2, qa, Co<double>{1.0, -1.0, 0.0, 1.0}, st);     // Mobius
-    outw_kernel<<<grid_for(N, 256), 256, 0, st>>>(qa, W.outw.as<double>(), n, Nloc, eps);
-    RUMB_LAUNCH("outw_kernel");
-    std::vector<ll> bounds;
-    const int *nodes = c.layer_table(n, bounds);
-    set_doubles_kernel<<<1, 32, 0, st>>>(W.mass.as<double>(), 1, 1.0);    // mass[empty set] = 1
-    RUMB_LAUNCH("set_doubles");
-    for (int cc = 1; cc <= n; ++cc) {
-        ll lo = bounds[cc], ns = bounds[cc + 1] - lo;
-        if (ns <= 0) continue;
-        mass_layer_kernel<<<grid_for(ns, 256), 256, 0, st>>>(qa, W.outw.as<double>(), W.mass.as<double>(),
-                                                             nodes + lo, ns, n, Nloc, eps);
-        RUMB_LAUNCH("mass_layer_kernel");
-    }
-    extract_kernel<<<grid_for(m2, 256), 256, 0, st>>>(qa, W.outw.as<double>(), W.mass.as<double>(), qb, n, Nloc,
-                                                      eps);
-    RUMB_LAUNCH("extract_kernel");
-    xf_transform<double, double>(n, qb, qa, Co<double>{1.0, 1.0, 0.0, 1.0}, st);  // zeta -> x_ub in qa
-    ub_eval_kernel<<<1, RED_THREADS, 0, st>>>(qa, W.obs.as<ll>(), pp, W.mp, W.pfit_cur.as<double>(), rr);
-    RUMB_LAUNCH("ub_eval_kernel");
-    if (pfit_best) {
-        ub_commit_kernel<<<grid_for(W.mp, 256), 256, 0, st>>>(W.pfit_cur.as<double>(), pfit_best, W.mp, rr);
-        RUMB_LAUNCH("ub_commit_kernel");
-    }
-    ub_best_kernel<<<1, 32, 0, st>>>(rr);
-    RUMB_LAUNCH("ub_best_kernel");
+struct CheckJob {
+    const T *x2 = nullptr;                 // iterates (slots of n 2^(n-1)); or the observed values y
+    const double *y = nullptr;
+    const double *p = nullptr;             // rows (slots of mp)
+    double *res = nullptr, *best = nullptr;
+    int slots = 1;
+    const int *active = nullptr, *lb = nullptr;
+    bool stats = true, with_lb = true, push = true;
+};
+
+template <class T>
+static CheckJob<T> solve_check(CertWork &W, const T *x2, bool with_lb) {
+    CheckJob<T> J;
+    J.x2 = x2;
+    J.p = W.p.as<double>();
+    J.res = W.res.as<double>();
+    J.best = W.pfit_best.as<double>();
+    J.with_lb = with_lb;
+    return J;
 }
 
-// phi (and the LB's residual sums); with_lb also scatters g and runs the longest path.
+// stats: phi; with_lb: the lower bound; push: x2 -> q = Mobius(x2) -> pushed masses -> zeta -> upper bound and
+// the running best (res; best may be null).
 template <class T>
-static void enqueue_stats_lb(Ctx &c, CertWork &W, int n, const T *x2, bool with_lb, cudaStream_t st,
-                             const double *p_ovr = nullptr, double *res_ovr = nullptr, const double *y_ovr = nullptr) {
-    const double *pp = p_ovr ? p_ovr : W.p.as<double>();
-    double *rr = res_ovr ? res_ovr : W.res.as<double>();
-    ll Nloc = 1LL << (n - 1), m2 = (ll)n * Nloc, N = 1LL << n;
-    double *g = W.qb.as<double>();
-    if (with_lb) RUMB_CUDA(cudaMemsetAsync(g, 0, (size_t)m2 * 8, st));
-    obs_stats_kernel<T><<<1, RED_THREADS, 0, st>>>(x2, W.obs.as<ll>(), pp, W.mp, with_lb ? g : nullptr, rr, y_ovr);
-    RUMB_LAUNCH("obs_stats_kernel");
-    if (!with_lb) return;
-    xf_transform<double, double>(n, g, g, Co<double>{1.0, 0.0, 1.0, 1.0}, st);    // subset sums
+static void enqueue_check(Ctx &c, CertWork &W, int n, const CheckJob<T> &J, cudaStream_t st) {
+    const ll Nloc = 1LL << (n - 1), m2 = (ll)n * Nloc, N = 1LL << n;
+    const unsigned K = (unsigned)J.slots;
+    CertArgs A{};
+    A.n = n; A.Nloc = Nloc; A.mp = W.mp;
+    A.qa = W.qa.as<double>(); A.qb = W.qb.as<double>();
+    A.outw = W.outw.as<double>(); A.mass = W.mass.as<double>(); A.dp = W.dp.as<double>();
+    A.obs = W.obs.as<ll>();
+    A.p = J.p; A.pfit = W.pfit_cur.as<double>(); A.best = J.best; A.res = J.res;
+    A.part = W.part.as<double>(); A.count = W.count.as<unsigned>();
+    A.pstride = W.mp;
+    A.active = J.active; A.lb = J.lb;
+    const bool lb = J.stats && J.with_lb;
+    if (lb) RUMB_CUDA(cudaMemsetAsync(A.qb, 0, (size_t)K * m2 * 8, st));
+    if (J.stats) {
+        obs_stats_kernel<T><<<dim3(32, K), 32, 0, st>>>(A, J.x2, m2, J.y, lb ? 1 : 0);
+        RUMB_LAUNCH("obs_stats_kernel");
+    }
+    if (lb) xf_transform<double, double>(n, A.qb, A.qb, Co<double>{1.0, 0.0, 1.0, 1.0}, st, J.slots, J.lb ? J.lb : J.active);
+    if (J.push) {
+        xf_transform<double, T>(n, J.x2, A.qa, Co<double>{1.0, -1.0, 0.0, 1.0}, st, J.slots, J.active);     // Mobius
+        outw_kernel<<<dim3(grid_for(N, 256), K), 256, 0, st>>>(A);
+        RUMB_LAUNCH("outw_kernel");
+    }
+    if (!lb && !J.push) return;
     std::vector<ll> bounds;
     const int *nodes = c.layer_table(n, bounds);
-    double *dp = W.dp.as<double>();
-    set_doubles_kernel<<<1, 32, 0, st>>>(dp, 1, 0.0);
-    RUMB_LAUNCH("set_doubles");
-    for (int cc = 1; cc <= n; ++cc) {
-        ll lo = bounds[cc], ns = bounds[cc + 1] - lo;
-        if (ns <= 0) continue;
-        lpath_layer_kernel<<<grid_for(ns, 256), 256, 0, st>>>(g, dp, nodes + lo, ns, n, Nloc);
-        RUMB_LAUNCH("lpath_layer_kernel");
+    if (n <= CERT_SMALL_N) {
+        cert_small_kernel<<<dim3(2, K), 1024, 0, st>>>(A, nodes, J.push ? 1 : 0, lb ? 1 : 0);
+        RUMB_LAUNCH("cert_small_kernel");
+    } else {
+        for (int cc = 1; cc <= n; ++cc) {
+            const ll lo = bounds[cc], ns = bounds[cc + 1] - lo;
+            const unsigned g = grid_for(ns, 128), mb = J.push ? g : 0;
+            cert_layer_kernel<<<dim3(mb + (lb ? g : 0), K), 128, 0, st>>>(A, nodes + lo, (int)ns, mb);
+            RUMB_LAUNCH("cert_layer_kernel");
+        }
     }
-    lb_final_kernel<<<1, 1, 0, st>>>(dp, N, rr);
-    RUMB_LAUNCH("lb_final_kernel");
+    if (!J.push) return;
+    extract_kernel<<<dim3(grid_for(m2, 256), K), 256, 0, st>>>(A);
+    RUMB_LAUNCH("extract_kernel");
+    xf_transform<double, double>(n, A.qb, A.qa, Co<double>{1.0, 1.0, 0.0, 1.0}, st, J.slots, J.active);  // zeta -> x_ub in qa
+    ub_eval_kernel<<<dim3(32, K), 32, 0, st>>>(A);
+    RUMB_LAUNCH("ub_eval_kernel");
+    if (A.best) {
+        ub_commit_kernel<<<dim3(grid_for(W.mp, 256), K), 256, 0, st>>>(A);
+        RUMB_LAUNCH("ub_commit_kernel");
+    }
 }
 
 // ================================================================= ADMM workspace
@@ -1143,12 +1039,10 @@ static bool run_leg_overlap(Ctx &c, CertWork &CW, BmWork<T> &W, const rumb_bm_pr
     T *x2s = W.snap.template as<T>();
     Graph h_ub, h_ublb;
     h_ub.capture(cs, [&] {
-        enqueue_stats_lb<T>(c, CW, n, x2s, false, cs);
-        enqueue_push<T>(c, CW, n, x2s, cs);
+        enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, false), cs);
     });
     h_ublb.capture(cs, [&] {
-        enqueue_stats_lb<T>(c, CW, n, x2s, true, cs);
-        enqueue_push<T>(c, CW, n, x2s, cs);
+        enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, true), cs);
     });
     struct AuxSync {   // no check may outlive the loop (its graphs and the snapshot)
         cudaStream_t s;
@@ -1236,12 +1130,10 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
     if (graphs) {
         g_iter.capture(st, [&] { enqueue_iterations<T>(W, C, n, st, chunk); });
         g_ub.capture(st, [&] {
-            enqueue_stats_lb<T>(c, CW, n, W.x2.template as<T>(), false, st);
-            enqueue_push<T>(c, CW, n, W.x2.template as<T>(), st);
+            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), false), st);
         });
         g_ublb.capture(st, [&] {
-            enqueue_stats_lb<T>(c, CW, n, W.x2.template as<T>(), true, st);
-            enqueue_push<T>(c, CW, n, W.x2.template as<T>(), st);
+            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), true), st);
         });
     }
     if (graphs && par.overlap_check) return run_leg_overlap<T>(c, CW, W, pr, par, L, t0, stall_exit, g_iter, chunk,
@@ -1271,8 +1163,7 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
         if (graphs) {
             (want_lb ? g_ublb : g_ub).launch(st);
         } else {
-            enqueue_stats_lb<T>(c, CW, n, W.x2.template as<T>(), want_lb, st);
-            enqueue_push<T>(c, CW, n, W.x2.template as<T>(), st);
+            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), want_lb), st);
         }
         RUMB_CUDA(cudaMemcpyAsync(res, CW.res.ptr, sizeof(res), cudaMemcpyDeviceToHost, st));
         unsigned int dev_err = 0;
@@ -1307,7 +1198,7 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
 
 // Device bytes of one solve, counted from the buffers it ensures: BmWork (9 slabs, the snapshot
 // slab, observation bits, per-menu observed masks, diagonal, error word) per state dtype, the
-// float64 certificate (2 slabs, 3 node arrays, 4 row arrays, result words), the popcount-ordered
+// float64 certificate (2 slabs, 3 node arrays, 4 row arrays, result words; not its 520 bytes of partial sums), the popcount-ordered
 // node ids and the uploaded rows.
 size_t bm_plan_bytes(int n, ll mp, int dtype) {
     if (n < 2 || n > 30) fail(RUMB_E_INVAL, "bm_plan: 2 <= n <= 30");
@@ -1522,15 +1413,13 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
         RUMB_CUDA(cudaStreamSynchronize(st));
         // one check first, so that its cached tables exist before the capture (no allocation inside)
         if (par->lb_every > 0) {
-            enqueue_stats_lb<T>(c, CW, n, W.x2.template as<T>(), true, st);
-            enqueue_push<T>(c, CW, n, W.x2.template as<T>(), st);
+            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), true), st);
             RUMB_CUDA(cudaStreamSynchronize(st));
         }
         auto body = [&] {
             enqueue_iterations<T>(W, C, n, st, iters);
             if (par->lb_every > 0) {
-                enqueue_stats_lb<T>(c, CW, n, W.x2.template as<T>(), true, st);
-                enqueue_push<T>(c, CW, n, W.x2.template as<T>(), st);
+                enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), true), st);
             }
         };
         // the profiled iterations and one check captured as a CUDA graph, as a solve replays them,
@@ -1636,7 +1525,7 @@ __global__ void scatter_rows_kernel(const ll *obs, const double *p, ll mp, doubl
 template <class T>
 struct BatchWork : public BmWorkBase {
     DevBuf x2, s, y, z, x, Ax, t1, t2, xhat;   // K slabs each
-    DevBuf obsbits, menu_obs, diag, err, active, p, res, pfit;
+    DevBuf obsbits, menu_obs, diag, err, active, lbf, p, res, pfit;
     int K = 0, n = 0;
     ll mp = 0;
     void ensure(int n_, ll mp_, int K_) {
@@ -1649,6 +1538,7 @@ struct BatchWork : public BmWorkBase {
         diag.ensure(64 * sizeof(T));
         err.ensure(16);
         active.ensure((size_t)K * 4);
+        lbf.ensure((size_t)K * 4);
         p.ensure((size_t)K * (size_t)mp * 8);
         pfit.ensure((size_t)K * (size_t)mp * 8);
         res.ensure((size_t)K * R_SLOTS * 8);
@@ -1686,6 +1576,12 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     if (!slot) slot.reset(new BatchWork<T>());
     BatchWork<T> &W = *static_cast<BatchWork<T> *>(slot.get());
     W.ensure(n, mp, K);
+    // slots checked together: as many as a quarter gigabyte of certificate arrays holds, and within a
+    // tenth of what is still free (one at a time needs no more than a single solve's)
+    RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
+    const size_t cert_budget = std::min<size_t>((size_t)256 << 20, fr / 10);
+    const int KC = (int)std::max<size_t>(1, std::min<size_t>((size_t)K, cert_budget / CertWork::slot_bytes(n, mp)));
+    CW.ensure(n, mp, KC);
     // shared structure: observed positions, bits, per-menu masks, diagonal
     DevProblem D;
     upload_problem(*pr, D, st);
@@ -1730,7 +1626,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
         ybuf.ensure((size_t)B * (size_t)mp * 8);
         RUMB_CUDA(cudaMemcpyAsync(ybuf.ptr, y0, (size_t)B * (size_t)mp * 8, cudaMemcpyHostToDevice, st));
     }
-    std::vector<int> act(K, 0), draw_of(K, -1);
+    std::vector<int> act(K, 0), lbf(K, 0), draw_of(K, -1);
     std::vector<ll> it_of(K, 0);
     std::vector<double> ub_of(K, INFINITY), lb_of(K, 0.0), phi_of(K, NAN);
     std::vector<int> nlb_of(K, 0), npush_of(K, 0);
@@ -1784,7 +1680,9 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
                 scatter_vals_kernel<T><<<grid_for(mp, 256), 256, 0, st>>>(CW.obs.as<ll>(), yb, mp, dst[0]);
                 RUMB_LAUNCH("scatter_vals_kernel");
             }
-            enqueue_stats_lb<T>(c, CW, n, dst[0], true, st, pk, rk, yb);
+            CheckJob<T> J;
+            J.y = yb; J.p = pk; J.res = rk; J.push = false;
+            enqueue_check<T>(c, CW, n, J, st);
             copy_double_kernel<<<1, 32, 0, st>>>(rk + R_LB_SEED, rk + R_LB_NOW);
             RUMB_LAUNCH("copy_double_kernel");
         }
@@ -1811,15 +1709,27 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
         for (int i = 0; i < par->check / chunk; ++i) g_iter.launch(st);
         int nact = 0;
         for (int k = 0; k < K; ++k) {
+            lbf[k] = act[k] && npush_of[k] % par->lb_every == 0;
             if (!act[k]) continue;
             ++nact;
             it_of[k] += par->check;
-            const T *x2k = I.x2 + (size_t)k * m2;
-            const double *pk = W.p.template as<double>() + (size_t)k * mp;
-            double *rk = W.res.template as<double>() + (size_t)k * R_SLOTS;
-            bool want_lb = (npush_of[k] % par->lb_every) == 0;
-            enqueue_stats_lb<T>(c, CW, n, x2k, want_lb, st, pk, rk);
-            enqueue_push<T>(c, CW, n, x2k, st, pk, rk, fit_out ? W.pfit.template as<double>() + (size_t)k * mp : nullptr);
+        }
+        if (par->lb_every > 1)
+            RUMB_CUDA(cudaMemcpyAsync(W.lbf.ptr, lbf.data(), (size_t)K * 4, cudaMemcpyHostToDevice, st));
+        for (int k = 0; k < K; k += KC) {
+            CheckJob<T> J;
+            J.slots = std::min(KC, K - k);
+            J.x2 = I.x2 + (size_t)k * m2;
+            J.p = W.p.template as<double>() + (size_t)k * mp;
+            J.res = W.res.template as<double>() + (size_t)k * R_SLOTS;
+            J.best = fit_out ? W.pfit.template as<double>() + (size_t)k * mp : nullptr;
+            J.active = I.active + k;
+            bool any = false, any_lb = false;
+            for (int q = k; q < k + J.slots; ++q) { any = any || act[q]; any_lb = any_lb || lbf[q]; }
+            if (!any) continue;
+            J.with_lb = any_lb;
+            J.lb = par->lb_every > 1 ? W.lbf.template as<int>() + k : nullptr;
+            enqueue_check<T>(c, CW, n, J, st);
         }
         total_iters += (ll)nact * par->check;
         RUMB_CUDA(cudaMemcpyAsync(res.data(), W.res.ptr, res.size() * 8, cudaMemcpyDeviceToHost, st));
@@ -2082,8 +1992,13 @@ int push_ub64_host(Ctx &c, int n, int dtype, const void *x, ll mp, const uint32_
     RUMB_CUDA(cudaMemcpyAsync(S.a.ptr, x, (size_t)m2 * es, cudaMemcpyHostToDevice, st));
     set_doubles_kernel<<<1, 32, 0, st>>>(CW.res.as<double>() + R_UB_BEST, 1, INFINITY);
     RUMB_LAUNCH("set_doubles");
-    if (dtype == RUMB_F64) enqueue_push<double>(c, CW, n, S.a.as<double>(), st);
-    else enqueue_push<float>(c, CW, n, S.a.as<float>(), st);
+    auto push = [&](auto *xs) {
+        auto J = solve_check(CW, xs, false);
+        J.stats = false;
+        enqueue_check(c, CW, n, J, st);
+    };
+    if (dtype == RUMB_F64) push((const double *)S.a.ptr);
+    else push((const float *)S.a.ptr);
     double res[R_SLOTS];
     RUMB_CUDA(cudaMemcpyAsync(res, CW.res.ptr, sizeof(res), cudaMemcpyDeviceToHost, st));
     if (p_fit) RUMB_CUDA(cudaMemcpyAsync(p_fit, CW.pfit_cur.ptr, (size_t)mp * 8, cudaMemcpyDeviceToHost, st));
@@ -2131,7 +2046,9 @@ int fw_lb64_host(Ctx &c, int n, ll mp, const uint32_t *menu, const int32_t *alt,
         if (hbad) fail(RUMB_E_INVAL, "an observed row's alternative is not in its menu or is out of range");
     }
     RUMB_CUDA(cudaMemcpyAsync(CW.p.ptr, D.d_p, (size_t)mp * 8, cudaMemcpyDeviceToDevice, st));
-    enqueue_stats_lb<double>(c, CW, n, S.a.as<double>(), true, st);
+    CheckJob<double> J = solve_check<double>(CW, S.a.as<double>(), true);
+    J.push = false;
+    enqueue_check<double>(c, CW, n, J, st);
     double res[R_SLOTS];
     RUMB_CUDA(cudaMemcpyAsync(res, CW.res.ptr, sizeof(res), cudaMemcpyDeviceToHost, st));
     RUMB_CUDA(cudaStreamSynchronize(st));
