@@ -100,6 +100,8 @@ int rumb_ctx_destroy(rumb_ctx *ctx) {
         if (ctx->c.ev_snap) cudaEventDestroy(ctx->c.ev_snap);
         if (ctx->c.ev_done) cudaEventDestroy(ctx->c.ev_done);
         if (ctx->c.res_host) cudaFreeHost(ctx->c.res_host);
+        if (ctx->c.ev_t0) cudaEventDestroy(ctx->c.ev_t0);
+        if (ctx->c.ev_t1) cudaEventDestroy(ctx->c.ev_t1);
         if (ctx->c.ev_a) cudaEventDestroy(ctx->c.ev_a);
         if (ctx->c.ev_b) cudaEventDestroy(ctx->c.ev_b);
         if (ctx->c.own) cudaStreamDestroy(ctx->c.own);

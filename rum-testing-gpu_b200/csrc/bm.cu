@@ -296,6 +296,7 @@ struct CertWork : public BmWorkBase {
     DevBuf pfit_cur, pfit_best;
     DevBuf res;               // R_SLOTS doubles
     DevBuf part, count;       // partial sums and finished CTAs
+    DevBuf menu, alt, rows, y, bad;   // a call's uploaded rows (and values y), their validity word
     ll mp = 0;
     int n = 0;
     static size_t slot_bytes(int n, ll mp) {
@@ -770,6 +771,7 @@ static void tune_iteration(Ctx &c, BmWork<T> &W, BmCoef &C, int n, cudaStream_t 
     auto it = c.tuned.find(key);
     if (it == c.tuned.end()) {
         BmCoef K = C;
+        enqueue_cold_start<T>(W, C, n, st);                  // a state to time on
         cudaEvent_t a, b;
         RUMB_CUDA(cudaEventCreate(&a));
         RUMB_CUDA(cudaEventCreate(&b));
@@ -839,25 +841,23 @@ static void tuned_or_default(Ctx &c, BmCoef &C, int n) {
 }
 
 // ----------------------------------------------------------------- problem upload
+// Device views of a call's rows: the caller's, or the certificate workspace's copies.
 struct DevProblem {
-    DevBuf menu, alt, p;
     const uint32_t *d_menu = nullptr;
     const int32_t *d_alt = nullptr;
     const double *d_p = nullptr;
 };
 
-static void upload_problem(const rumb_bm_problem &pr, DevProblem &D, cudaStream_t st) {
-    if (pr.on_device) {
-        D.d_menu = pr.menu; D.d_alt = pr.alt; D.d_p = pr.p;
-        return;
-    }
-    D.menu.ensure((size_t)pr.mp * 4);
-    D.alt.ensure((size_t)pr.mp * 4);
-    D.p.ensure((size_t)pr.mp * 8);
-    RUMB_CUDA(cudaMemcpyAsync(D.menu.ptr, pr.menu, (size_t)pr.mp * 4, cudaMemcpyHostToDevice, st));
-    RUMB_CUDA(cudaMemcpyAsync(D.alt.ptr, pr.alt, (size_t)pr.mp * 4, cudaMemcpyHostToDevice, st));
-    RUMB_CUDA(cudaMemcpyAsync(D.p.ptr, pr.p, (size_t)pr.mp * 8, cudaMemcpyHostToDevice, st));
-    D.d_menu = D.menu.as<uint32_t>(); D.d_alt = D.alt.as<int32_t>(); D.d_p = D.p.as<double>();
+static DevProblem upload_problem(const rumb_bm_problem &pr, CertWork &W, cudaStream_t st) {
+    W.bad.ensure(4);
+    if (pr.on_device) return DevProblem{pr.menu, pr.alt, pr.p};
+    W.menu.ensure((size_t)pr.mp * 4);
+    W.alt.ensure((size_t)pr.mp * 4);
+    W.rows.ensure((size_t)pr.mp * 8);
+    RUMB_CUDA(cudaMemcpyAsync(W.menu.ptr, pr.menu, (size_t)pr.mp * 4, cudaMemcpyHostToDevice, st));
+    RUMB_CUDA(cudaMemcpyAsync(W.alt.ptr, pr.alt, (size_t)pr.mp * 4, cudaMemcpyHostToDevice, st));
+    RUMB_CUDA(cudaMemcpyAsync(W.rows.ptr, pr.p, (size_t)pr.mp * 8, cudaMemcpyHostToDevice, st));
+    return DevProblem{W.menu.as<uint32_t>(), W.alt.as<int32_t>(), W.rows.as<double>()};
 }
 
 // observations -> obs positions + p (cert workspace), xhat + obsbits (ADMM workspace of dtype T)
@@ -866,8 +866,7 @@ static void setup_obs(Ctx &c, CertWork &CW, BmWork<T> *W, const rumb_bm_problem 
                       cudaStream_t st) {
     int n = pr.n;
     ll Nloc = 1LL << (n - 1), m2 = (ll)n * Nloc;
-    DevBuf bad;
-    bad.ensure(4);
+    DevBuf &bad = CW.bad;
     RUMB_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, st));
     DevBuf tmpx, tmpb;
     T *xhat;
@@ -999,6 +998,48 @@ struct Graph {
     }
 };
 
+// The graphs of one kind of solve (state dtype; single or batched), kept with the context: capturing and
+// instantiating them again for every solve of a session or a bootstrap took 0.3-0.5 ms, and up to 100 ms
+// when the driver was busy. They hold no input: the rows and states they work on are uploaded into the
+// workspaces whose addresses, with every launch parameter, are the key; another key captures again.
+struct SolveGraphs : public BmWorkBase {
+    std::vector<unsigned long long> key;
+    Graph iter, ub, ublb, side_ub, side_ublb;
+    void use(std::vector<unsigned long long> k) {
+        if (k == key) return;
+        for (Graph *g : {&iter, &ub, &ublb, &side_ub, &side_ublb}) g->reset();
+        key = std::move(k);
+    }
+};
+static SolveGraphs &solve_graphs(std::unique_ptr<BmWorkBase> &slot) {
+    if (!slot) slot.reset(new SolveGraphs());
+    return *static_cast<SolveGraphs *>(slot.get());
+}
+static void key_add(std::vector<unsigned long long> &k, double v) {
+    unsigned long long b;
+    memcpy(&b, &v, 8);
+    k.push_back(b);
+}
+static void key_add(std::vector<unsigned long long> &k, const void *p) { k.push_back((unsigned long long)(uintptr_t)p); }
+template <class T>
+static std::vector<unsigned long long> graph_key(Ctx &c, const CertWork &CW, const IterPtrs<T> &I, const BmCoef &C, int n,
+                                                 int chunk, const void *snap) {
+    std::vector<unsigned long long> k{(unsigned long long)n, (unsigned long long)CW.mp, (unsigned long long)chunk,
+                                      (unsigned long long)C.lo_bits, (unsigned long long)C.prox_form,
+                                      (unsigned long long)C.fuse, (unsigned long long)C.dr, (unsigned long long)I.slots};
+    for (double v : {C.b1, C.b2, C.alpha, C.p}) key_add(k, v);
+    for (const void *p : {(const void *)I.x2, (const void *)I.s, (const void *)I.y, (const void *)I.z, (const void *)I.x,
+                          (const void *)I.Ax, (const void *)I.t1, (const void *)I.t2, (const void *)I.xhat,
+                          (const void *)I.diag, (const void *)I.menu_obs, (const void *)I.err, (const void *)I.active, snap})
+        key_add(k, p);
+    for (const DevBuf *b : {&CW.qa, &CW.qb, &CW.outw, &CW.mass, &CW.dp, &CW.obs, &CW.p, &CW.pfit_cur, &CW.pfit_best, &CW.res,
+                            &CW.part, &CW.count})
+        key_add(k, (const void *)b->ptr);
+    std::vector<ll> bounds;
+    key_add(k, (const void *)c.layer_table(n, bounds));
+    return k;
+}
+
 static int graph_chunk(int check) {
     int k = 1;
     for (int d = 1; d <= 32 && d <= check; ++d)
@@ -1029,21 +1070,18 @@ struct LoopState {
 template <class T>
 static bool run_leg_overlap(Ctx &c, CertWork &CW, BmWork<T> &W, const rumb_bm_problem &pr,
                             const rumb_bm_params &par, LoopState &L, Clock::time_point t0, bool stall_exit,
-                            Graph &g_iter, int chunk, rumb_trace_fn trace, void *user) {
+                            SolveGraphs &G, int chunk, rumb_trace_fn trace, void *user) {
     const int n = pr.n;
     const ll m2 = (ll)n << (n - 1);
     cudaStream_t st = c.own;
     c.ensure_aux();
     cudaStream_t cs = c.aux;
-    W.snap.ensure((size_t)m2 * sizeof(T));
     T *x2s = W.snap.template as<T>();
-    Graph h_ub, h_ublb;
-    h_ub.capture(cs, [&] {
-        enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, false), cs);
-    });
-    h_ublb.capture(cs, [&] {
-        enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, true), cs);
-    });
+    Graph &g_iter = G.iter;
+    Graph &h_ub = G.side_ub, &h_ublb = G.side_ublb;
+    if (par.lb_every > 1 && !h_ub.e)
+        h_ub.capture(cs, [&] { enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, false), cs); });
+    if (!h_ublb.e) h_ublb.capture(cs, [&] { enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2s, true), cs); });
     struct AuxSync {   // no check may outlive the loop (its graphs and the snapshot)
         cudaStream_t s;
         ~AuxSync() { cudaStreamSynchronize(s); }
@@ -1125,20 +1163,23 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
     int n = pr.n;
     cudaStream_t st = c.own;
     int chunk = graph_chunk(par.check);
-    Graph g_iter, g_ub, g_ublb;
-    bool graphs = par.use_graph != 0;
+    SolveGraphs &G = solve_graphs(sizeof(T) == 8 ? c.graphs64 : c.graphs32);
+    Graph &g_iter = G.iter, &g_ub = G.ub, &g_ublb = G.ublb;
+    const bool graphs = par.use_graph != 0, overlap = graphs && par.overlap_check;
     if (graphs) {
-        g_iter.capture(st, [&] { enqueue_iterations<T>(W, C, n, st, chunk); });
-        g_ub.capture(st, [&] {
-            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), false), st);
-        });
-        g_ublb.capture(st, [&] {
-            enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), true), st);
-        });
+        if (overlap) W.snap.ensure(((size_t)n << (n - 1)) * sizeof(T));
+        G.use(graph_key<T>(c, CW, iter_ptrs<T>(W), C, n, chunk, overlap ? W.snap.ptr : nullptr));
+        if (!g_iter.e) g_iter.capture(st, [&] { enqueue_iterations<T>(W, C, n, st, chunk); });
     }
-    if (graphs && par.overlap_check) return run_leg_overlap<T>(c, CW, W, pr, par, L, t0, stall_exit, g_iter, chunk,
-                                                              trace, user);
-    double res[R_SLOTS];
+    if (overlap) return run_leg_overlap<T>(c, CW, W, pr, par, L, t0, stall_exit, G, chunk, trace, user);
+    if (graphs) {
+        const T *x2 = W.x2.template as<T>();
+        if (par.lb_every > 1 && !g_ub.e)
+            g_ub.capture(st, [&] { enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2, false), st); });
+        if (!g_ublb.e) g_ublb.capture(st, [&] { enqueue_check<T>(c, CW, n, solve_check<T>(CW, x2, true), st); });
+    }
+    double *res = c.res_host;                              // pinned: the copies are queued behind the check
+    unsigned int *dev_err = reinterpret_cast<unsigned int *>(c.res_host + R_SLOTS);
     while (L.it < par.max_iter) {
         if (graphs) {
             for (int i = 0; i < par.check / chunk; ++i) g_iter.launch(st);
@@ -1165,11 +1206,10 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
         } else {
             enqueue_check<T>(c, CW, n, solve_check<T>(CW, W.x2.template as<T>(), want_lb), st);
         }
-        RUMB_CUDA(cudaMemcpyAsync(res, CW.res.ptr, sizeof(res), cudaMemcpyDeviceToHost, st));
-        unsigned int dev_err = 0;
-        RUMB_CUDA(cudaMemcpyAsync(&dev_err, W.err.ptr, 4, cudaMemcpyDeviceToHost, st));
+        RUMB_CUDA(cudaMemcpyAsync(res, CW.res.ptr, R_SLOTS * sizeof(double), cudaMemcpyDeviceToHost, st));
+        RUMB_CUDA(cudaMemcpyAsync(dev_err, W.err.ptr, 4, cudaMemcpyDeviceToHost, st));
         RUMB_CUDA(cudaStreamSynchronize(st));
-        if (dev_err) fail(RUMB_E_TIMEOUT, "a kernel's bounded wait for its TMA copies gave up");
+        if (*dev_err) fail(RUMB_E_TIMEOUT, "a kernel's bounded wait for its TMA copies gave up");
         L.push_s += secs(tp, Clock::now());
         L.checks++;
         L.phi = std::sqrt(res[R_PHI2]);
@@ -1228,16 +1268,13 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     cudaStream_t st = c.own;
     c.cancel.store(0);
     c.join_in();
-    cudaEvent_t e0, e1;
-    RUMB_CUDA(cudaEventCreate(&e0));
-    RUMB_CUDA(cudaEventCreate(&e1));
-    struct EvGuard { cudaEvent_t a, b; ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); } } eg{e0, e1};
+    c.ensure_host();
+    cudaEvent_t e0 = c.ev_t0, e1 = c.ev_t1;
     RUMB_CUDA(cudaEventRecord(e0, st));
 
     CertWork &CW = cert_work(c);
     CW.ensure(n, pr->mp);
-    DevProblem D;
-    upload_problem(*pr, D, st);
+    const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     bool use32 = par->dtype != RUMB_F64;
     BmWork<double> *W64 = nullptr;
@@ -1253,14 +1290,8 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     if (W64) RUMB_CUDA(cudaMemcpyAsync(W64->diag.ptr, C.diag.data(), C.diag.size() * 8, cudaMemcpyHostToDevice, st));
     // transform split (tuned once per context, n and dtype), then the initial state
     BmCoef C64 = C;
-    if (W32) {
-        enqueue_cold_start<float>(*W32, C, n, st);
-        tune_iteration<float>(c, *W32, C, n, st);
-    }
-    if (W64) {
-        enqueue_cold_start<double>(*W64, C64, n, st);
-        tune_iteration<double>(c, *W64, C64, n, st);
-    }
+    if (W32) tune_iteration<float>(c, *W32, C, n, st);
+    if (W64) tune_iteration<double>(c, *W64, C64, n, st);
     if (!W32) C = C64;
     if (use32) {
         if (warm) copy_state_in<float>(*W32, *warm, m2, st);
@@ -1336,8 +1367,7 @@ int bm_iterate(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, voi
     c.join_in();
     CertWork &CW = cert_work(c);
     CW.ensure(n, pr->mp);
-    DevProblem D;
-    upload_problem(*pr, D, st);
+    const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     auto run = [&](auto tag) {
         using T = decltype(tag);
@@ -1391,8 +1421,7 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
     c.join_in();
     CertWork &CW = cert_work(c);
     CW.ensure(n, pr->mp);
-    DevProblem D;
-    upload_problem(*pr, D, st);
+    const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     Prof prof;
     prof.st = st;
@@ -1405,7 +1434,6 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
         RUMB_CUDA(cudaMemsetAsync(W.err.ptr, 0, 16, st));
         std::vector<T> dg(C.diag.begin(), C.diag.end());
         RUMB_CUDA(cudaMemcpyAsync(W.diag.ptr, dg.data(), dg.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        enqueue_cold_start<T>(W, C, n, st);
         tune_iteration<T>(c, W, C, n, st);
         enqueue_cold_start<T>(W, C, n, st);
         enqueue_begin<T>(iter_ptrs<T>(W), C, n, st);
@@ -1525,7 +1553,7 @@ __global__ void scatter_rows_kernel(const ll *obs, const double *p, ll mp, doubl
 template <class T>
 struct BatchWork : public BmWorkBase {
     DevBuf x2, s, y, z, x, Ax, t1, t2, xhat;   // K slabs each
-    DevBuf obsbits, menu_obs, diag, err, active, lbf, p, res, pfit;
+    DevBuf obsbits, menu_obs, diag, err, active, lbf, p, res, pfit, draws, fits;
     int K = 0, n = 0;
     ll mp = 0;
     void ensure(int n_, ll mp_, int K_) {
@@ -1561,7 +1589,6 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     auto t0 = Clock::now();
     // slots by memory
     size_t fr = 0, tot = 0;
-    RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
     double frac = (bp && bp->mem_fraction > 0) ? bp->mem_fraction : 0.8;
     size_t per = batch_slot_bytes<T>(n, mp);
     CertWork &CW = cert_work(c);
@@ -1577,18 +1604,15 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     BatchWork<T> &W = *static_cast<BatchWork<T> *>(slot.get());
     W.ensure(n, mp, K);
     // slots checked together: as many as a quarter gigabyte of certificate arrays holds, and within a
-    // tenth of what is still free (one at a time needs no more than a single solve's)
-    RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
-    const size_t cert_budget = std::min<size_t>((size_t)256 << 20, fr / 10);
+    // tenth of what the states leave free (one at a time needs no more than a single solve's)
+    const size_t cert_budget = std::min<size_t>((size_t)256 << 20, (fr - std::min(fr, (size_t)K * per)) / 10);
     const int KC = (int)std::max<size_t>(1, std::min<size_t>((size_t)K, cert_budget / CertWork::slot_bytes(n, mp)));
     CW.ensure(n, mp, KC);
     // shared structure: observed positions, bits, per-menu masks, diagonal
-    DevProblem D;
-    upload_problem(*pr, D, st);
+    const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     {
-        DevBuf bad;
-        bad.ensure(4);
+        DevBuf &bad = CW.bad;
         RUMB_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, st));
         RUMB_CUDA(cudaMemsetAsync(W.xhat.ptr, 0, (size_t)m2 * sizeof(T) * K, st));
         RUMB_CUDA(cudaMemsetAsync(W.obsbits.ptr, 0, (size_t)((m2 + 31) / 32) * 4, st));
@@ -1616,12 +1640,14 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     I.active = W.active.template as<int>();
     // the schedule tuned on a single-draw workspace, when known
     tuned_or_default<T>(c, C, n);
-    DevBuf pbuf;                                    // the draws' rows, uploaded once
-    pbuf.ensure((size_t)B * (size_t)mp * 8);
+    // the draws' rows, uploaded once; kept with the workspace up to 64 MB
+    const size_t row_bytes = (size_t)B * (size_t)mp * 8;
+    DevBuf own_p, own_y;
+    DevBuf &pbuf = row_bytes <= ((size_t)64 << 20) ? W.draws : own_p, &ybuf = row_bytes <= ((size_t)64 << 20) ? W.fits : own_y;
+    pbuf.ensure(row_bytes);
     RUMB_CUDA(cudaMemcpyAsync(pbuf.ptr, P, (size_t)B * (size_t)mp * 8, cudaMemcpyHostToDevice, st));
     const double *y0 = bp ? bp->y0 : nullptr;       // predicted fits: a lower-bound seed per draw
     double *fit_out = bp ? bp->p_fit : nullptr;
-    DevBuf ybuf;
     if (y0) {
         ybuf.ensure((size_t)B * (size_t)mp * 8);
         RUMB_CUDA(cudaMemcpyAsync(ybuf.ptr, y0, (size_t)B * (size_t)mp * 8, cudaMemcpyHostToDevice, st));
@@ -1695,13 +1721,13 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     RUMB_CUDA(cudaStreamSynchronize(st));
     auto t_setup = Clock::now();
     const int chunk = graph_chunk(par->check);
-    Graph g_iter;
-    g_iter.capture(st, [&] { enqueue_iterations_ptrs<T>(I, C, n, st, chunk); });
+    SolveGraphs &G = solve_graphs(sizeof(T) == 8 ? c.batch_graphs64 : c.batch_graphs32);
+    G.use(graph_key<T>(c, CW, I, C, n, chunk, nullptr));
+    Graph &g_iter = G.iter;
+    if (!g_iter.e) g_iter.capture(st, [&] { enqueue_iterations_ptrs<T>(I, C, n, st, chunk); });
     std::vector<double> res((size_t)K * R_SLOTS);
-    cudaEvent_t e0, e1;
-    RUMB_CUDA(cudaEventCreate(&e0));
-    RUMB_CUDA(cudaEventCreate(&e1));
-    struct EvGuard { cudaEvent_t a, b; ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); } } eg{e0, e1};
+    c.ensure_host();
+    cudaEvent_t e0 = c.ev_t0, e1 = c.ev_t1;
     RUMB_CUDA(cudaEventRecord(e0, st));
     while (done < B) {
         if (c.cancel.load()) fail(RUMB_E_CANCEL, "cancelled");
@@ -1983,8 +2009,7 @@ int push_ub64_host(Ctx &c, int n, int dtype, const void *x, ll mp, const uint32_
     c.join_in();
     CertWork &CW = cert_work(c);
     CW.ensure(n, mp);
-    DevProblem D;
-    upload_problem(pr, D, st);
+    const DevProblem D = upload_problem(pr, CW, st);
     setup_obs<double>(c, CW, nullptr, pr, D, st);
     Scratch &S = scratch(c);
     size_t es = dtype == RUMB_F64 ? 8 : 4;
@@ -2019,20 +2044,18 @@ int fw_lb64_host(Ctx &c, int n, ll mp, const uint32_t *menu, const int32_t *alt,
     c.join_in();
     CertWork &CW = cert_work(c);
     CW.ensure(n, mp);
-    DevProblem D;
-    upload_problem(pr, D, st);
+    const DevProblem D = upload_problem(pr, CW, st);
     // the y slab: scatter y at the observed positions through the xhat path (xhat := y)
-    rumb_bm_problem py = pr;
-    py.p = y;
-    DevProblem Dy;
-    upload_problem(py, Dy, st);
+    CW.y.ensure((size_t)mp * 8);
+    RUMB_CUDA(cudaMemcpyAsync(CW.y.ptr, y, (size_t)mp * 8, cudaMemcpyHostToDevice, st));
+    DevProblem Dy = D;
+    Dy.d_p = CW.y.as<double>();
     Scratch &S = scratch(c);
     S.a.ensure((size_t)m2 * 8);
     S.d.ensure((size_t)((m2 + 31) / 32) * 4);
     // positions with xhat = y
     {
-        DevBuf bad;
-        bad.ensure(4);
+        DevBuf &bad = CW.bad;
         RUMB_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, st));
         RUMB_CUDA(cudaMemsetAsync(S.a.ptr, 0, (size_t)m2 * 8, st));
         RUMB_CUDA(cudaMemsetAsync(S.d.ptr, 0, (size_t)((m2 + 31) / 32) * 4, st));

@@ -29,10 +29,14 @@ struct Ctx {
     std::unique_ptr<BmWorkBase> batch64, batch32;  // batched-draw workspaces
     std::unique_ptr<BmWorkBase> cert;           // float64 certificate workspace
     std::unique_ptr<BmWorkBase> scratch;        // primitive calls' scratch
+    // the captured iteration and check graphs of the last solve of each kind (bm.cu); after the workspaces
+    // they launch on, so that they go first
+    std::unique_ptr<BmWorkBase> graphs64, graphs32, batch_graphs64, batch_graphs32;
+    cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;   // a call's device time (made on first use)
     // the iteration's tuned schedule per (n, state bytes): transform low-window size, prox form,
     // fused passes (0 / 1)
     std::map<std::pair<int, int>, std::array<int, 3>> tuned;
-    // overlapped checks: a second stream, its two events and pinned result words (made on first use)
+    // overlapped checks: a second stream and its two events; a check's pinned result words (made on first use)
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_snap = nullptr, ev_done = nullptr;
     double *res_host = nullptr;
@@ -41,7 +45,12 @@ struct Ctx {
         RUMB_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
         RUMB_CUDA(cudaEventCreateWithFlags(&ev_snap, cudaEventDisableTiming));
         RUMB_CUDA(cudaEventCreateWithFlags(&ev_done, cudaEventDisableTiming));
-        RUMB_CUDA(cudaMallocHost(&res_host, 64 * sizeof(double)));
+    }
+    // pinned words for a check's results and the timing events
+    void ensure_host() {
+        if (!res_host) RUMB_CUDA(cudaMallocHost(&res_host, 64 * sizeof(double)));
+        if (!ev_t0) RUMB_CUDA(cudaEventCreate(&ev_t0));
+        if (!ev_t1) RUMB_CUDA(cudaEventCreate(&ev_t1));
     }
 
     // Make the context's stream wait for the caller's stream (call start) ...

@@ -585,7 +585,11 @@ def _is_oom(e):
 
 def _machine_line():
     try:
-        free, total = context().mem_info()
-        return "GPU 0 (%.0f GB, librumb %d)" % (total / 1e9, __import__("rumb._lib")._lib.load().rumb_version())
+        # the size of a context's memory does not change: asked of the driver once (on a shared machine
+        # the query took 5 to 130 ms now and then, after solves of 11 ms)
+        ctx = context()
+        if getattr(ctx, "total_bytes", None) is None:
+            ctx.total_bytes = ctx.mem_info()[1]
+        return "GPU 0 (%.0f GB, librumb %d)" % (ctx.total_bytes / 1e9, __import__("rumb._lib")._lib.load().rumb_version())
     except Exception:
         return "no GPU"
