@@ -126,6 +126,14 @@ inline bool pdl_enabled() {
     return on;
 }
 
+// While one of these lives, the calling thread's launch_pdl launches in plain stream order.
+inline thread_local int g_plain_order = 0;
+struct PlainOrder {
+    bool on;
+    explicit PlainOrder(bool plain) : on(plain) { g_plain_order += on; }
+    ~PlainOrder() { g_plain_order -= on; }
+};
+
 template <class... KArgs, class... Args>
 inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -135,7 +143,7 @@ inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() && g_plain_order == 0 ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cuda_check(cudaLaunchKernelEx(&cfg, kern, args...), "cudaLaunchKernelEx");
