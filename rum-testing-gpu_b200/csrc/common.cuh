@@ -113,9 +113,11 @@ inline void smem_optin(K *kernel, int bytes, std::atomic<unsigned long long> &do
 // then waits until the kernel before it has completed and its writes are visible. Because every
 // kernel so launched waits before it can complete, completion stays ordered down the stream.
 // RUMB_PDL=0 launches them in plain stream order.
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_grid_sync() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch_next();
+    pdl_wait();
 }
 
 inline bool pdl_enabled() {

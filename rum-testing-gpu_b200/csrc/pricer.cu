@@ -57,6 +57,7 @@ struct PricerArgs {
     float *mcur, *ecur;
     uint8_t *pred;             // nullptr when this layer keeps no predecessors
     unsigned int *layer_step;  // float bits, atomicMax (steps are >= 0)
+    unsigned int *bcnt;        // per quantization block: its finished CTAs (zero between launches), or nullptr
     // mask mode: the layer's nodes, values and predecessors indexed by the mask
     const int *nodes;
     float *vmask;
@@ -148,13 +149,25 @@ __device__ __forceinline__ float w_scan(const ull *menus, const float *scores, l
     return w;
 }
 
-// w(x, D) from pair p's cover list (sx = x's first score).
+// w(x, D) from pair p's cover list (sx = x's first score): eight entries and then their scores in flight
+// together, added in list order (the chain entry -> score -> add is what a layer of lists with tens of
+// entries waits for).
 template <class IT>
 __device__ __forceinline__ float w_list(const unsigned *offs, const IT *ent, ull p, const float *sx) {
     const unsigned b = __ldg(offs + p), e = __ldg(offs + p + 1);
+    constexpr int U = 8;
     float w = 0.0f;
-#pragma unroll 4
-    for (unsigned i = b; i < e; ++i) w = __fadd_rn(w, __ldg(sx + __ldg(ent + i)));
+    for (unsigned i = b; i < e; i += U) {
+        unsigned id[U];
+        float sc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) id[u] = i + u < e ? (unsigned)__ldg(ent + i + u) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) sc[u] = i + u < e ? __ldg(sx + id[u]) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i + u < e) w = __fadd_rn(w, sc[u]);
+    }
     return w;
 }
 
@@ -164,6 +177,67 @@ __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in
     if (!in) return 0.0f;
     if (A.wmode == W_LIST16) return w_list(A.loffs, (const uint16_t *)A.lent, p, A.scores + lo);
     return w_list(A.loffs, (const uint32_t *)A.lent, p, A.scores + lo);
+}
+
+// Quantizes block blk (1024 ranks) of a layer with `nt` threads (a multiple of 32): block min / max, step =
+// (max - min) / levels, q = rintf((v - min) / step). The values were written by this or other CTAs.
+__device__ __forceinline__ void quant_block(const PricerArgs &A, const float *vals, ull blk, int tid, int nt) {
+    __shared__ float smin[32], smax[32];
+    const ull r0 = blk * PB, end = r0 + PB < A.count ? r0 + PB : A.count;
+    float tmin = 3.0e38f, tmax = -3.0e38f;
+    for (ull r = r0 + tid; r < end; r += nt) {
+        const float v = __ldcg(vals + r);
+        tmin = fminf(tmin, v);
+        tmax = fmaxf(tmax, v);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+    }
+    if ((tid & 31) == 0) { smin[tid >> 5] = tmin; smax[tid >> 5] = tmax; }
+    __syncthreads();
+    float bmin = smin[0], bmax = smax[0];
+    for (int i = 1; i < nt / 32; ++i) { bmin = fminf(bmin, smin[i]); bmax = fmaxf(bmax, smax[i]); }
+    const float levels = A.mode == 2 ? 65535.0f : 16777215.0f;
+    const float step = __fdiv_rn(__fsub_rn(bmax, bmin), levels);
+    if (tid == 0) {
+        A.mcur[blk] = bmin;
+        A.ecur[blk] = step;
+        atomicMax(A.layer_step, __float_as_uint(step));
+    }
+    for (ull r = r0 + tid; r < end; r += nt) {
+        const float v = __ldcg(vals + r);
+        float q = (step > 0.0f) ? rintf(__fdiv_rn(__fsub_rn(v, bmin), step)) : 0.0f;
+        q = fminf(fmaxf(q, 0.0f), levels);
+        const unsigned int qi = (unsigned int)q;
+        if (A.mode == 2) {
+            A.vcur_h[r] = (uint16_t)qi;
+        } else {
+            A.vcur_h[r] = (uint16_t)(qi >> 8);
+            A.lcur[r] = (uint8_t)(qi & 255u);
+        }
+    }
+}
+
+// The end of a layer kernel's CTA that wrote ranks [r0, r0 + span) (span divides 1024): the last CTA of a
+// quantization block quantizes it, so that a layer is one launch (a launch of its own took 4 us of a layer's
+// 10 to 25 at n = 18). Every thread of the CTA calls it.
+__device__ __forceinline__ void finish_block(const PricerArgs &A, const float *vals, ull r0, int span) {
+    if (A.mode < 2 || !A.bcnt) return;
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    const ull blk = r0 / PB;
+    if (threadIdx.x == 0) {
+        const ull first = blk * PB, cnt = A.count - first < PB ? A.count - first : PB;
+        const unsigned parts = (unsigned)((cnt + span - 1) / span);
+        last = atomicAdd(A.bcnt + blk, 1u) + 1u == parts;
+        if (last) A.bcnt[blk] = 0u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    quant_block(A, vals, blk, (int)threadIdx.x, (int)blockDim.x);
 }
 
 // One popcount layer k of the sweep.
@@ -181,16 +255,22 @@ __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in
 //   stream: D is the colex unranking of r; the value of D \ {x} is read from the previous layer's
 //         storage at its colex rank; output: the float32 value (f32 mode, and the predecessor
 //         byte) or the value for stream_quant_kernel to quantize (u16 / u24).
-// stream_quant_kernel: one CTA per quantization block of 1024 ranks, as the number format asks:
-// block min / max, step, rintf quantization of every value (u16 / u24 modes).
+// Quantization blocks are 1024 ranks, as the number format asks (u16 / u24 modes): the last CTA of a block
+// quantizes it (finish_block), or stream_quant_kernel after the group sweep.
 constexpr int PE_R = 128, PE_G = 8;
 static_assert((PE_R / 32) * PE_G == 32 && (PE_G & (PE_G - 1)) == 0, "32 warps; PE_G a power of two");
 // Layers whose 128-rank CTAs would not give every SM two of them run 32 ranks per CTA (8 warps).
 constexpr int PE_R_SMALL = 32;
 
+//
+// The sums w(x, D) do not depend on the layer before, only its values do: a layer's CTAs form their sums
+// from the pricer's lists and the call's scores (both complete before the sweep's first layer
+// started) while the layers before still run, and wait for them only then. The layers are chains of
+// dependent loads on a few hundred CTAs, so they overlap almost whole: a u24 sweep at n = 18 (0.5 % of the
+// menus) 403 -> 300 us.
 template <bool MASK, int PR>
 __global__ void __launch_bounds__(PR * PE_G) layer_eval_kernel(PricerArgs A, float *vals) {
-    pdl_grid_sync();                                       // launched by launch_pdl
+    pdl_launch_next();                                     // launched by launch_pdl
     static_assert(PR % 32 == 0 && (PR / 32) * PE_G <= 32, "at most 32 warps");
     __shared__ float pbest[PE_G][PR];
     __shared__ signed char pbx[PE_G][PR];
@@ -208,41 +288,51 @@ __global__ void __launch_bounds__(PR * PE_G) layer_eval_kernel(PricerArgs A, flo
     ull D = 0;
     if (valid) D = MASK ? (ull)(unsigned)A.nodes[r] : colex_unrank(r, k, n, sbin);
     const ull pbase = A.lbase + r * (ull)k;
+    constexpr int XM = (MAXN_PR + PE_G - 1) / PE_G;          // x = xg, xg + 8, ... of this thread
+    float wsum[XM];
+#pragma unroll
+    for (int q = 0; q < XM; ++q) {
+        const int x = xg + PE_G * q;
+        wsum[q] = 0.0f;
+        if (x >= n) continue;                                // uniform per warp
+        const bool in = valid && ((D >> x) & 1ULL);
+        wsum[q] = w_of(A, x, D, in, pbase + __popcll(D & ((1ULL << x) - 1ULL)));
+    }
+    pdl_wait();
     float best = 0.0f;
     int bestx = -1;
-    for (int x = n - 1; x >= 0; --x) {
-        if ((x & (PE_G - 1)) != xg) continue;            // uniform per warp
-        const bool in = valid && ((D >> x) & 1ULL);
-        const int j = __popcll(D & ((1ULL << x) - 1ULL));
-        const float wsum = w_of(A, x, D, in, pbase + j);
-        if (in) {
-            float prev;
-            if (MASK) prev = A.vmask[D ^ (1ULL << x)];
-            else prev = decode_prev(A, colex_rank_without(r, D, x, j, n, sbin));
-            const float cand = __fadd_rn(prev, wsum);
-            if (bestx < 0 || cand >= best) { best = cand; bestx = x; }
-        }
+#pragma unroll
+    for (int q = XM - 1; q >= 0; --q) {
+        const int x = xg + PE_G * q;
+        if (x >= n || !valid || !((D >> x) & 1ULL)) continue;
+        float prev;
+        if (MASK) prev = A.vmask[D ^ (1ULL << x)];
+        else prev = decode_prev(A, colex_rank_without(r, D, x, __popcll(D & ((1ULL << x) - 1ULL)), n, sbin));
+        const float cand = __fadd_rn(prev, wsum[q]);
+        if (bestx < 0 || cand >= best) { best = cand; bestx = x; }
     }
     pbest[xg][loc] = best;
     pbx[xg][loc] = (signed char)bestx;
     __syncthreads();
-    if (xg != 0 || !valid) return;
-    float b = pbest[0][loc];
-    int bx = pbx[0][loc];
-    for (int g = 1; g < PE_G; ++g) {
-        const float c = pbest[g][loc];
-        const int cx = pbx[g][loc];
-        if (cx < 0) continue;
-        if (bx < 0 || c > b || (c == b && cx < bx)) { b = c; bx = cx; }
+    if (xg == 0 && valid) {
+        float b = pbest[0][loc];
+        int bx = pbx[0][loc];
+        for (int g = 1; g < PE_G; ++g) {
+            const float c = pbest[g][loc];
+            const int cx = pbx[g][loc];
+            if (cx < 0) continue;
+            if (bx < 0 || c > b || (c == b && cx < bx)) { b = c; bx = cx; }
+        }
+        if (MASK) {
+            A.vmask[D] = b;
+            A.pmask[D] = (uint8_t)bx;
+        } else {
+            if (A.pred) A.pred[r] = (uint8_t)bx;
+            if (A.mode == 1) A.vcur_f[r] = b;
+            else vals[r] = b;
+        }
     }
-    if (MASK) {
-        A.vmask[D] = b;
-        A.pmask[D] = (uint8_t)bx;
-        return;
-    }
-    if (A.pred) A.pred[r] = (uint8_t)bx;
-    if (A.mode == 1) A.vcur_f[r] = b;
-    else vals[r] = b;
+    if (!MASK) finish_block(A, vals, (ull)blockIdx.x * PR, PR);
 }
 
 // The float64 max sweep (sweep_max64, the Frank-Wolfe bound's longest path when the float64 slab
@@ -319,13 +409,13 @@ __global__ void __launch_bounds__(PR * PE_G) max64_layer_kernel(PricerArgs A, co
 // candidates then merge in x order with `>` (ties -> lowest x).
 template <bool MASK, class IT>
 __global__ void __launch_bounds__(1024) layer_wide_kernel(PricerArgs A, float *vals) {
-    pdl_grid_sync();                                       // launched by launch_pdl
+    pdl_launch_next();                                     // launched by launch_pdl; the sums come before the wait
     __shared__ ull sbin[MASK ? 1 : BIN_MAX];
     __shared__ float cv[MAXN_PR];
     __shared__ ull sD;
     const int n = A.n, k = A.k;
     const ull r = blockIdx.x;
-    const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int x = threadIdx.x >> 5, lane = threadIdx.x & 31;   // a warp per alternative (lists: n <= 26)
     if (!MASK) stage_binom(sbin, A.binom, n);
     __syncthreads();
     if (threadIdx.x == 0) sD = MASK ? (ull)(unsigned)A.nodes[r] : colex_unrank(r, k, n, sbin);
@@ -333,12 +423,12 @@ __global__ void __launch_bounds__(1024) layer_wide_kernel(PricerArgs A, float *v
     const ull D = sD;
     const ull pbase = A.lbase + r * (ull)k;
     const IT *ent = (const IT *)A.lent;
-    for (int x = w; x < n; x += nw) {
-        if (!((D >> x) & 1ULL)) continue;                 // uniform per warp
-        const int j = __popcll(D & ((1ULL << x) - 1ULL));
+    const bool in = x < n && ((D >> x) & 1ULL);               // uniform per warp
+    const int j = __popcll(D & ((1ULL << x) - 1ULL));
+    float wsum = 0.0f;
+    if (in) {
         const unsigned b = __ldg(A.loffs + pbase + j), e = __ldg(A.loffs + pbase + j + 1);
         const float *sx = A.scores + A.offsets[x];
-        float wsum = 0.0f;
         float v = (b + lane < e) ? __ldg(sx + __ldg(ent + b + lane)) : 0.0f;
         for (unsigned c = b; c < e; c += 32) {
             const unsigned nx = c + 32 + lane;
@@ -347,28 +437,31 @@ __global__ void __launch_bounds__(1024) layer_wide_kernel(PricerArgs A, float *v
             for (int u = 0; u < m; ++u) wsum = __fadd_rn(wsum, __shfl_sync(0xffffffffu, v, u));
             v = vn;
         }
-        if (lane == 0) {
-            const float prev = MASK ? A.vmask[D ^ (1ULL << x)]
-                                    : decode_prev(A, colex_rank_without(r, D, x, j, n, sbin));
-            cv[x] = __fadd_rn(prev, wsum);
-        }
+    }
+    pdl_wait();
+    if (in && lane == 0) {
+        const float prev = MASK ? A.vmask[D ^ (1ULL << x)]
+                                : decode_prev(A, colex_rank_without(r, D, x, j, n, sbin));
+        cv[x] = __fadd_rn(prev, wsum);
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    float best = 0.0f;
-    int bx = -1;
-    for (int x = 0; x < n; ++x) {
-        if (!((D >> x) & 1ULL)) continue;
-        if (bx < 0 || cv[x] > best) { best = cv[x]; bx = x; }
+    if (threadIdx.x == 0) {
+        float best = 0.0f;
+        int bx = -1;
+        for (int x = 0; x < n; ++x) {
+            if (!((D >> x) & 1ULL)) continue;
+            if (bx < 0 || cv[x] > best) { best = cv[x]; bx = x; }
+        }
+        if (MASK) {
+            A.vmask[D] = best;
+            A.pmask[D] = (uint8_t)bx;
+        } else {
+            if (A.pred) A.pred[r] = (uint8_t)bx;
+            if (A.mode == 1) A.vcur_f[r] = best;
+            else vals[r] = best;
+        }
     }
-    if (MASK) {
-        A.vmask[D] = best;
-        A.pmask[D] = (uint8_t)bx;
-        return;
-    }
-    if (A.pred) A.pred[r] = (uint8_t)bx;
-    if (A.mode == 1) A.vcur_f[r] = best;
-    else vals[r] = best;
+    if (!MASK) finish_block(A, vals, r, 1);
 }
 
 // Cover-list construction, once per pricer: thread per subset D (mask order, all layers in one
@@ -414,36 +507,22 @@ __global__ void stream_decode_kernel(PricerArgs A, ull count_prev, float *dec) {
 
 __global__ void __launch_bounds__(PB) stream_quant_kernel(PricerArgs A, const float *vals) {
     pdl_grid_sync();                                       // launched by launch_pdl
-    __shared__ float smin[PB / 32], smax[PB / 32];
-    const ull r = (ull)blockIdx.x * PB + threadIdx.x;
-    const bool valid = r < A.count;
-    const float best = valid ? vals[r] : 0.0f;
-    float tmin = valid ? best : 3.0e38f, tmax = valid ? best : -3.0e38f;
-    for (int o = 16; o > 0; o >>= 1) {
-        tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
-        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-    }
-    if ((threadIdx.x & 31) == 0) { smin[threadIdx.x >> 5] = tmin; smax[threadIdx.x >> 5] = tmax; }
-    __syncthreads();
-    float bmin = smin[0], bmax = smax[0];
-    for (int i = 1; i < PB / 32; ++i) { bmin = fminf(bmin, smin[i]); bmax = fmaxf(bmax, smax[i]); }
-    const float levels = A.mode == 2 ? 65535.0f : 16777215.0f;
-    float step = __fdiv_rn(__fsub_rn(bmax, bmin), levels);
-    if (threadIdx.x == 0) {
-        A.mcur[blockIdx.x] = bmin;
-        A.ecur[blockIdx.x] = step;
-        atomicMax(A.layer_step, __float_as_uint(step));
-    }
-    if (!valid) return;
-    float q = (step > 0.0f) ? rintf(__fdiv_rn(__fsub_rn(best, bmin), step)) : 0.0f;
-    q = fminf(fmaxf(q, 0.0f), levels);
-    unsigned int qi = (unsigned int)q;
-    if (A.mode == 2) {
-        A.vcur_h[r] = (uint16_t)qi;
+    quant_block(A, vals, blockIdx.x, (int)threadIdx.x, PB);
+}
+
+// Layer 0 (V[empty set] = 0: q 0, offset 0, step 0) and no steps yet, before a sweep of the stream storage.
+__global__ void stream_start_kernel(PricerArgs A, unsigned int *steps) {
+    const int i = threadIdx.x;
+    if (i <= A.n) steps[i] = 0u;
+    if (i != 0) return;
+    if (A.mode == 1) {
+        A.vcur_f[0] = 0.0f;
     } else {
-        A.vcur_h[r] = (uint16_t)(qi >> 8);
-        A.lcur[r] = (uint8_t)(qi & 255u);
+        A.vcur_h[0] = 0;
+        if (A.mode == 3) A.lcur[0] = 0;
     }
+    A.mcur[0] = 0.0f;
+    A.ecur[0] = 0.0f;
 }
 
 // Result block written by the device backtrace (one small D2H copy per price call).
@@ -457,6 +536,7 @@ struct PriceOut {
     ull node;              // descent only: the node reached at layer k_pred
 };
 
+constexpr int BT_SMALL_K = 9;
 // Descent through the stored predecessor layers (stream modes), then the mask DP on the
 // sub-lattice of the node reached; one CTA. V/pred scratch: 2^K entries (K = k_pred); Ws: the
 // 2^K K sub-lattice sums. descend_only: stop after the descent and leave the node and the number
@@ -470,17 +550,33 @@ __global__ void backtrace_kernel(int n, int k_pred, const ull *binom, uint8_t *c
     __shared__ int elems[MAXN_PR];
     __shared__ int spos;
     __shared__ ull sbin[BIN_MAX];
+    __shared__ const uint8_t *spred[MAXN_PR + 1];
+    // the sub-lattice's arrays on the SM while they are small: every round of its DP waits for them
+    __shared__ float sV[1 << BT_SMALL_K], sW[(1 << BT_SMALL_K) * BT_SMALL_K];
+    __shared__ uint8_t sP[1 << BT_SMALL_K];
     stage_binom(sbin, binom, n);
+    for (int k = threadIdx.x; k <= n; k += blockDim.x) spred[k] = preds[k];
+    if (k_pred <= BT_SMALL_K) {
+        Vs = sV;
+        Ps = sP;
+        Ws = sW;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         ull D = (n >= 64) ? ~0ULL : ((1ULL << n) - 1ULL);
+        const int lane = threadIdx.x;
         int pos = 0;
         for (int k = n; k > k_pred; --k) {
-            ull r = colex_rank_dev(D, sbin, n);
-            int x = preds[k][r];
-            out->rank_pos[x] = pos++;
+            ull r = 0;                                       // D's colex rank, a lane per bit (and its bit + 32)
+            for (int b = lane; b < n; b += 32)
+                if ((D >> b) & 1ULL) r += sbin[b * (n + 1) + __popcll(D & ((2ULL << b) - 1ULL))];
+            for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            const int x = spred[k][r];
+            if (lane == 0) out->rank_pos[x] = pos;
+            ++pos;
             D ^= 1ULL << x;
         }
+        if (lane == 0) {
         int K = 0;
         for (int b = 0; b < n; ++b)
             if ((D >> b) & 1ULL) elems[K++] = b;
@@ -493,6 +589,7 @@ __global__ void backtrace_kernel(int n, int k_pred, const ull *binom, uint8_t *c
             out->qtop = q;
             out->mtop = mtop[0];
             out->etop = etop[0];
+        }
         }
     }
     __syncthreads();
@@ -1156,6 +1253,7 @@ struct Pricer {
     std::vector<std::unique_ptr<DevBuf>> pred;   // per layer >= k_pred
     DevBuf pred_ptrs;                       // device array of pred pointers (n+1)
     DevBuf layer_step;                      // n+1 uints (float bits)
+    DevBuf bcnt;                            // per quantization block: finished CTAs (quantized storage)
     DevBuf Vs, Ps;                          // sub-lattice / mask scratch
     DevBuf Ws;                              // sub-lattice sums w(x_j, D(s)): 2^k_pred * k_pred floats
     DevBuf vals;                            // a layer's float32 values before quantization
@@ -1509,6 +1607,10 @@ Pricer *pricer_create(Ctx &c, int n, ll mp, const uint64_t *menus, const int64_t
             P->m[i].ensure((size_t)nblk * 4);
             P->e[i].ensure((size_t)nblk * 4);
         }
+        if (mode >= 2) {
+            P->bcnt.ensure((size_t)nblk * 4);
+            RUMB_CUDA(cudaMemsetAsync(P->bcnt.ptr, 0, (size_t)nblk * 4, st));
+        }
         std::vector<uint8_t *> ptrs(n + 1, nullptr);
         P->pred.resize(n + 1);
         for (int k = P->k_pred; k <= n; ++k) {
@@ -1640,7 +1742,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             RUMB_LAUNCH("layer_eval_kernel");
         };
         auto wide_kernel = [&]() {
-            const unsigned threads = 32u * (unsigned)std::min(n, 32), grid = (unsigned)A.count;
+            const unsigned threads = 32u * (unsigned)n, grid = (unsigned)A.count;   // with lists n <= 26
             if (mask && P->wmode == W_LIST16) launch_pdl(layer_wide_kernel<true, uint16_t>, dim3(grid), dim3(threads), 0, st, A, vals);
             else if (mask) launch_pdl(layer_wide_kernel<true, uint32_t>, dim3(grid), dim3(threads), 0, st, A, vals);
             else if (P->wmode == W_LIST16) launch_pdl(layer_wide_kernel<false, uint16_t>, dim3(grid), dim3(threads), 0, st, A, vals);
@@ -1650,7 +1752,7 @@ static void run_sweep(Pricer *P, const float *scores) {
         if (P->wmode != W_SCAN && P->wide[A.k]) wide_kernel();
         else thread_kernel();
     };
-    RUMB_CUDA(cudaMemsetAsync(P->layer_step.ptr, 0, (size_t)(n + 1) * 4, st));
+    if (P->by_mask) RUMB_CUDA(cudaMemsetAsync(P->layer_step.ptr, 0, (size_t)(n + 1) * 4, st));
     auto args = [&](int k) {
         PricerArgs A{};
         A.n = n;
@@ -1691,11 +1793,16 @@ static void run_sweep(Pricer *P, const float *scores) {
         RUMB_LAUNCH("mask_readout_kernel");
     } else {
         int cur = 0, prev = 1;
-        // layer 0: V = 0 (offset 0, step 0, q 0)
-        RUMB_CUDA(cudaMemsetAsync(P->v[prev].ptr, 0, P->mode == 1 ? 4 : 2, st));
-        if (P->mode == 3) RUMB_CUDA(cudaMemsetAsync(P->l[prev].ptr, 0, 1, st));
-        RUMB_CUDA(cudaMemsetAsync(P->m[prev].ptr, 0, 4, st));
-        RUMB_CUDA(cudaMemsetAsync(P->e[prev].ptr, 0, 4, st));
+        {
+            PricerArgs A = args(0);
+            A.vcur_f = P->v[prev].as<float>();
+            A.vcur_h = P->v[prev].as<uint16_t>();
+            A.lcur = P->l[prev].as<uint8_t>();
+            A.mcur = P->m[prev].as<float>();
+            A.ecur = P->e[prev].as<float>();
+            stream_start_kernel<<<1, 64, 0, st>>>(A, P->layer_step.as<unsigned int>());
+            RUMB_LAUNCH("stream_start_kernel");
+        }
         std::vector<ull> bh, b10;
         if (P->stream_group) {
             b10 = binom_host(SG_LOW);
@@ -1720,6 +1827,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             A.ecur = P->e[cur].as<float>();
             A.pred = k >= P->k_pred ? P->pred[k]->as<uint8_t>() : nullptr;
             A.layer_step = P->layer_step.as<unsigned int>() + k;
+            if (!P->stream_group) A.bcnt = P->bcnt.as<unsigned int>();
             if (P->stream_group) {
                 const int hb = n - SG_LOW;
                 StreamGroupArgs G{};
@@ -1746,7 +1854,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             } else {
                 layer(A, false, P->vals.as<float>());
             }
-            if (A.mode != 1) {
+            if (A.mode != 1 && P->stream_group) {
                 launch_pdl(stream_quant_kernel, dim3((unsigned)((A.count + PB - 1) / PB)), dim3(PB), 0, st, A, P->vals.as<float>());
                 RUMB_LAUNCH("stream_quant_kernel");
             }
