@@ -373,13 +373,29 @@ __global__ void mse_grad_kernel(const float *out, const float *T, const int *idx
     if (threadIdx.x == 0) loss_parts[blockIdx.x] = red[0];
 }
 
-// db[n] = sum over rows of the bf16 gradient G [Mb x N] (one thread per column, fixed row order)
-__global__ void colsum_kernel(const bf16 *G, int Mb, int N, float *db) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+// db[n] = sum over rows of the bf16 gradient G [Mb x N]: a CTA takes 32 columns, warp g the rows g, g + 32, ...
+// (64-byte reads, eight in flight), then the 32 partial sums of a column are added in warp order: a fixed order
+// for a fixed Mb. One thread per column walking all rows took 67 us at 1024 x 1024.
+constexpr int CS_U = 8;
+__global__ void __launch_bounds__(1024) colsum_kernel(const bf16 *G, int Mb, int N, float *db) {
+    __shared__ float part[32][33];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int r = 0; r < Mb; ++r) s += __bfloat162float(G[(ll)r * N + n]);
-    db[n] = s;
+    if (n < N)
+        for (int r0 = g; r0 < Mb; r0 += 32 * CS_U) {
+            float v[CS_U];
+#pragma unroll
+            for (int u = 0; u < CS_U; ++u) v[u] = r0 + 32 * u < Mb ? __bfloat162float(G[(ll)(r0 + 32 * u) * N + n]) : 0.f;
+#pragma unroll
+            for (int u = 0; u < CS_U; ++u) s += v[u];
+        }
+    part[g][lane] = s;
+    __syncthreads();
+    if (g != 0 || n >= N) return;
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t += part[i][lane];
+    db[n] = t;
 }
 
 // Adam on f32 master weights; writes the bf16 copy [R x Cc] and its transpose [Cc x R]
@@ -593,7 +609,7 @@ static void backward(Mlp &m, cudaStream_t st) {
         g.C = y.gW.as<float>();
         g.err = m.err.as<unsigned int>();
         gemm(GT->as<bf16>(), m.XT[l].as<bf16>(), g, st);
-        colsum_kernel<<<grid_for(y.outp, 128), 128, 0, st>>>(G->as<bf16>(), m.Mb, y.outp, y.gb.as<float>());
+        colsum_kernel<<<grid_for(y.outp, 32), 1024, 0, st>>>(G->as<bf16>(), m.Mb, y.outp, y.gb.as<float>());
         RUMB_LAUNCH("colsum_kernel");
         if (l == 0) break;
         // G_{l-1} = (G W_l) * gelu'(Z_{l-1}) : A = G [Mb x outp], B = W_l^T [inp x outp]
