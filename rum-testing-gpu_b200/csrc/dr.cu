@@ -506,12 +506,12 @@ __global__ void __launch_bounds__(NT, 512 / NT) dr_high_kernel(DrArgs P, int M) 
 }
 
 // ---------------------------------------------------------------- middle passes
-// Window [s0, s0 + B) of both streams in place, one column per thread; s0 = s_mid - 1 for the
-// alternatives below M. BEFORE the high window: Q^T on a and Q^T A' on e; after it: Q on a, A Q on e.
+// Window [s0, s0 + B) of both streams in place, one column of one stream (blockIdx.z: a, e) per thread; s0 =
+// s_mid - 1 for the alternatives below M. BEFORE the high window: Q^T on a and Q^T A' on e; after it: Q on a,
+// A Q on e. Bound by HBM: 6.1-6.4 TB/s.
 template <int B, bool BEFORE>
 __global__ void __launch_bounds__(256) dr_mid_kernel(DrArgs P, int M, int s_mid) {
     if (P.active && !P.active[blockIdx.y]) return;
-    const ll o = (ll)blockIdx.y * P.bstride;
     constexpr int R = 1 << B;
     const ll per = P.Nloc >> B;                              // columns of one alternative
     const ll i = blockIdx.x * (ll)blockDim.x + threadIdx.x;
@@ -519,25 +519,20 @@ __global__ void __launch_bounds__(256) dr_mid_kernel(DrArgs P, int M, int s_mid)
     if (x >= P.n) return;
     const int s0 = x < M ? s_mid - 1 : s_mid;
     const ll r = i - x * per, low = r & ((1LL << s0) - 1);
-    const ll p0 = o + x * P.Nloc + ((r >> s0) << (s0 + B)) + low;
-    double v[R], w[R];
+    double *p = (blockIdx.z ? P.e : P.a) + (ll)blockIdx.y * P.bstride + x * P.Nloc + ((r >> s0) << (s0 + B)) + low;
+    double v[R];
 #pragma unroll
-    for (int j = 0; j < R; ++j) {
-        v[j] = P.a[p0 + ((ll)j << s0)];
-        w[j] = P.e[p0 + ((ll)j << s0)];
-    }
-    xf_regs<double, R, 0, B, XF_UNIT>(v, P.kQ);
-    if (BEFORE) {
-        xf_regs<double, R, 0, B, XF_APRIME>(w, P.kAp);
-        xf_regs<double, R, 0, B, XF_UNIT>(w, P.kQ);
+    for (int j = 0; j < R; ++j) v[j] = p[(ll)j << s0];
+    if (blockIdx.z == 0) {
+        xf_regs<double, R, 0, B, XF_UNIT>(v, P.kQ);
+    } else if (BEFORE) {
+        xf_regs<double, R, 0, B, XF_APRIME>(v, P.kAp);
+        xf_regs<double, R, 0, B, XF_UNIT>(v, P.kQ);
     } else {
-        xf_regs<double, R, 0, B, XF_GEN>(w, P.kAQ);
+        xf_regs<double, R, 0, B, XF_GEN>(v, P.kAQ);
     }
 #pragma unroll
-    for (int j = 0; j < R; ++j) {
-        P.a[p0 + ((ll)j << s0)] = v[j];
-        P.e[p0 + ((ll)j << s0)] = w[j];
-    }
+    for (int j = 0; j < R; ++j) p[(ll)j << s0] = v[j];
 }
 
 // ---------------------------------------------------------------- into and out of the iteration
@@ -612,23 +607,23 @@ __global__ void dr_end_kernel(const double *c, double *x2, double *s, double *y,
 
 // ---------------------------------------------------------------- launchers
 // The windows of n alternatives: tiles of 2^M menus, a high window of BH bits (BH + 1 for the
-// alternatives below M) and `mid` bits left to middle passes. A low tile holds its n runs of v in
-// shared memory and three CTAs share an SM, a high tile holds 2^(BH + 1) rows of at least four values:
-// M = 7, 8, 9 keep both sides near n / 2 up to n = 20 (measured in us per iteration with check and
-// graph, M = 7 / 8 / 9: n = 14 15.2 / 16.6 / -, n = 16 23.5 / 20.8 / -, n = 18 - / 52.0 / 56.5, n = 19 - /
-// 124.6 / 123.4, n = 20 - / - / 267). Beyond that eight high bits and middle passes are the faster side:
-// a 12-bit high window leaves one CTA per SM.
+// alternatives below M) and `mid` bits left to middle passes of up to 5 bits. A low tile holds its n runs of v
+// in shared memory and three CTAs share an SM, a high tile holds 2^(BH + 1) rows of at least four values: without
+// middle passes up to 10 high bits, with them eight (12 high bits leave one CTA per SM). M = 8 has the faster low
+// kernel (n = 18 34.5 us against 39.6 with M = 9, n = 21 274 / 328, n = 22 576 / 667), M = 7 below n = 15 (an
+// iteration at n = 14 15.2 us against 16.6, at n = 16 23.5 against 20.8 with M = 8); M = 9 is taken where it
+// saves a middle pass (n = 20: 249 us an iteration against 320, n = 23, 28), and at n = 19, where M = 8's high
+// tiles would have 32-byte rows (116 us against 118).
 struct DrShape {
     int M, BH, mid;
 };
+static int dr_mid_bits(int n, int M) { return n - 1 - M <= 10 ? 0 : n - 1 - M - 8; }
 static DrShape dr_shape(int n) {
+    auto passes = [&](int M) { return (dr_mid_bits(n, M) + 4) / 5; };
     DrShape S{};
-    S.M = n >= 19 ? 9 : n >= 15 ? 8 : 7;
-    S.BH = n - 1 - S.M;
-    if (S.BH > 10) {
-        S.mid = S.BH - 8;
-        S.BH = 8;
-    }
+    S.M = n < 15 ? 7 : n == 19 || passes(9) < passes(8) ? 9 : 8;
+    S.mid = dr_mid_bits(n, S.M);
+    S.BH = n - 1 - S.M - S.mid;
     return S;
 }
 
@@ -663,7 +658,8 @@ template <bool OUT>
 static void dr_low(const DrArgs &P, int M, int slots, cudaStream_t st) {
     if (M == 7) dr_low_go<7, 256, 16, OUT>(P, slots, st);
     else if (M == 8 && P.n <= 16) dr_low_go<8, 256, 16, OUT>(P, slots, st);
-    else if (M == 8) dr_low_go<8, 128, 32, OUT>(P, slots, st);
+    else if (M == 8 && P.n <= 18) dr_low_go<8, 128, 32, OUT>(P, slots, st);   // n = 18: 34.5 us against 36
+    else if (M == 8) dr_low_go<8, 256, 32, OUT>(P, slots, st);                // n = 22: 576 us against 612
     else dr_low_go<9, 256, 32, OUT>(P, slots, st);
 }
 
@@ -682,15 +678,16 @@ static void dr_high_go(const DrArgs &P, int M, int slots, cudaStream_t st) {
 template <bool BEFORE>
 static void dr_mid(const DrArgs &P, const DrShape &S, int slots, cudaStream_t st) {
     for (int s = S.M, left = S.mid; left > 0;) {
-        const int B = left > 8 ? 4 : left > 4 ? (left + 1) / 2 : left;   // 2^B values of both streams in registers
+        const int passes = (left + 4) / 5, B = (left + passes - 1) / passes;
         const ll cols = ((ll)P.n * P.Nloc) >> B;
-        const dim3 grid(grid_for(cols, 256), (unsigned)slots);
+        const dim3 grid(grid_for(cols, 256), (unsigned)slots, 2);
         dr_prof(BEFORE ? "dr_mid_before<f64>" : "dr_mid_after<f64>", P, slots, 4.0, st);
         switch (B) {
             case 1: dr_launch(dr_mid_kernel<1, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
             case 2: dr_launch(dr_mid_kernel<2, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
             case 3: dr_launch(dr_mid_kernel<3, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
-            default: dr_launch(dr_mid_kernel<4, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
+            case 4: dr_launch(dr_mid_kernel<4, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
+            default: dr_launch(dr_mid_kernel<5, BEFORE>, grid, dim3(256), 0, st, P, S.M, s); break;
         }
         RUMB_LAUNCH("dr_mid_kernel");
         prof_end(st);

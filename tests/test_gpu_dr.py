@@ -1,5 +1,5 @@
 """The two-kernel float64 iteration (csrc/dr.cu) against the oracle at every window shape: one and two
-high-window exchanges (n = 13..20), middle passes (n = 21), both p_hat lane groups (n <= 16 and
+high-window exchanges (n = 13..20), middle passes (n = 21, 22), both p_hat lane groups (n <= 16 and
 above), menus without, with some and with all members observed, and start states that no iteration
 leaves behind (s and y both positive, x2 off the simplex)."""
 import numpy as np
@@ -18,7 +18,7 @@ def _rows(n):
     return m[keep], a[keep], p[keep]
 
 
-@pytest.mark.parametrize("n", [13, 14, 15, 16, 17, 18, 19, 20, 21])
+@pytest.mark.parametrize("n", [13, 14, 15, 16, 17, 18, 19, 20, 21, 22])
 def test_two_kernel_iteration_tracks_oracle(ctx, n):
     menu, alt, p = _rows(n)
     O.set_threads(0)
