@@ -671,11 +671,11 @@ static void enqueue_iterations_ptrs(const IterPtrs<T> &I, const BmCoef &C, int n
             return;
         }
     }
-    // Two windows and more (n >= 14) go out in plain stream order: a CTA launched ahead waits on its SM
-    // beside the kernel before. float32, us an iteration ahead / plain: n = 14 13.7 / 11.8, n = 15 17.5 / 14.5, n = 16
-    // 23.9 / 20.9, n = 17 31.1 / 29.3, n = 18 55.4 / 55.6, n = 20 236 / 233, n = 22 1,287 / 1,227; with one
-    // window launching ahead is the faster side or equal (n = 11 7.2 / 7.6, n = 13 10.8 / 11.3).
-    PlainOrder order(n >= 14);
+    // From n = 11 they go out in plain stream order: a CTA launched ahead waits on its SM beside the kernel
+    // before. us an iteration ahead / plain: float32 n = 11 7.3 / 7.0, n = 13 10.6 / 10.4, n = 15 17.5 / 14.5, n = 16
+    // 23.9 / 20.9, n = 17 31.1 / 29.3, n = 18 55.4 / 55.6, n = 20 236 / 233, n = 22 1,287 / 1,227, float64 n = 12
+    // 10.5 / 9.6; up to n = 10 launching ahead is even or the faster side (float64 n = 8 5.08 / 5.32).
+    PlainOrder order(n >= 11);
     for (int i = 0; i < count; ++i) enqueue_iteration_ptrs<T>(I, C, n, st, i, count);
 }
 
