@@ -1,6 +1,5 @@
-// BM-ADMM on the Block-Marschak slab (sm_100a): the fused per-menu prox, the float64
-// certificate (feasibility push -> upper bound, Frank-Wolfe longest path -> lower bound) and the
-// certified solve loop.
+// BM-ADMM on the Block-Marschak slab (sm_100a): the cold start's prox, the sequences of iteration
+// kernels, the check's launches (cert.cuh) and the certified solve loop, single and batched.
 //
 // Reference behaviour (mingxiz/rum-testing-gpu):
 //   iteration        solver/bm_admm/solver.py:33-54 (_EW_SRC), :240-254 (one_iter)
@@ -11,13 +10,11 @@
 //   push (UB)        solver/common/transforms.py:94-98, solver/common/arcflow_kernels.py:357-434
 //   Frank-Wolfe LB   solver/common/transforms.py:101-114, solver/common/arcflow_kernels.py:388-448
 //
-// Per iteration this runs 4 butterflies (A', Q^T with the eigen-space diagonal fused into its
-// last store, Q, A) with the w / rhs elementwise steps fused into the A' loads and stores, and
-// ONE prox kernel that also does the over-relaxed point, the z update, the s/y update with its
-// nonnegativity clamp and the x2 copy (the reference's fuse_xk, prox_all, fuse_z, fuse_sy and
-// copyto). The prox walks menus in mask order, so a warp's members of one alternative are 32
-// consecutive entries of that alternative's block (coalesced), and projects with Michelot's
-// active-set iteration in registers instead of an insertion sort.
+// float64 states of n >= DR_MIN_N iterate in the two kernels of dr.cu. The others (float32, smaller lattices,
+// pinned forms) run 4 butterflies (A', Q^T with the eigen-space diagonal fused into its last store, Q, A) as
+// transform passes (xform.cuh) with the w / rhs and s / y steps fused into their loads and stores, and one prox
+// kernel (prox.cu) that also does the over-relaxed point, the z update and the x2 copy (the reference's
+// fuse_xk, prox_all, fuse_z, fuse_sy and copyto).
 #include <atomic>
 #include <chrono>
 #include <cstring>
@@ -302,7 +299,8 @@ struct CertWork : public BmWorkBase {
     static size_t slot_bytes(int n, ll mp) {
         return 2 * 8 * ((size_t)n << (n - 1)) + 3 * ((size_t)8 << n) + 8 * (size_t)mp + CERT_PART * 8 + 8;
     }
-    void ensure(int n_, ll mp_, int slots = 1) {
+    // st: the stream whose work uses the arrays (the counters are zeroed on it)
+    void ensure(int n_, ll mp_, cudaStream_t st, int slots = 1) {
         n = n_;
         mp = mp_;
         const size_t m2 = (size_t)n << (n - 1), N = (size_t)1 << n, K = (size_t)slots;
@@ -319,7 +317,7 @@ struct CertWork : public BmWorkBase {
         part.ensure(K * CERT_PART * 8);
         if (count.bytes < K * 8) {
             count.ensure(K * 8);
-            RUMB_CUDA(cudaMemset(count.ptr, 0, K * 8));
+            RUMB_CUDA(cudaMemsetAsync(count.ptr, 0, K * 8, st));
         }
     }
 };
@@ -1278,7 +1276,7 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     RUMB_CUDA(cudaEventRecord(e0, st));
 
     CertWork &CW = cert_work(c);
-    CW.ensure(n, pr->mp);
+    CW.ensure(n, pr->mp, c.own);
     const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     bool use32 = par->dtype != RUMB_F64;
@@ -1316,15 +1314,16 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     auto t_setup = Clock::now();
 
     LoopState L;
-    bool final_dtype64 = !use32;
+    bool final_dtype64 = !use32, iterated64 = !use32;
     if (use32) {
         // a float32 state stops at its rounding floor: mixed hands over to float64, float32 ends
         bool stall_exit = par->dtype == RUMB_MIXED || par->stall_checks > 0;
         bool done = run_leg<float>(c, CW, *W32, C, *pr, *par, L, t0, stall_exit, trace, user);
         if (!done && par->dtype == RUMB_MIXED) {
             promote_state(*W32, *W64, m2, st);
-            enqueue_begin<double>(iter_ptrs<double>(*W64), C64, n, st);
             final_dtype64 = true;
+            iterated64 = L.it < par->max_iter;           // else the promoted state is the final one
+            if (iterated64) enqueue_begin<double>(iter_ptrs<double>(*W64), C64, n, st);
             run_leg<double>(c, CW, *W64, C64, *pr, *par, L, t0, false, trace, user);
         } else if (!done) {
             L.stop = RUMB_STOP_STALL;
@@ -1336,7 +1335,7 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     if (p_fit && std::isfinite(L.ub))
         RUMB_CUDA(cudaMemcpyAsync(p_fit, CW.pfit_best.ptr, (size_t)pr->mp * 8, cudaMemcpyDeviceToHost, st));
     if (keep) {
-        if (final_dtype64) enqueue_end<double>(iter_ptrs<double>(*W64), C64, n, st);
+        if (iterated64) enqueue_end<double>(iter_ptrs<double>(*W64), C64, n, st);
         *keep = final_dtype64 ? copy_state_out<double>(*W64, n, c.device, st)
                               : copy_state_out<float>(*W32, n, c.device, st);
     }
@@ -1371,7 +1370,7 @@ int bm_iterate(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, voi
     cudaStream_t st = c.own;
     c.join_in();
     CertWork &CW = cert_work(c);
-    CW.ensure(n, pr->mp);
+    CW.ensure(n, pr->mp, c.own);
     const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     auto run = [&](auto tag) {
@@ -1425,7 +1424,7 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
     cudaStream_t st = c.own;
     c.join_in();
     CertWork &CW = cert_work(c);
-    CW.ensure(n, pr->mp);
+    CW.ensure(n, pr->mp, c.own);
     const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
     Prof prof;
@@ -1597,7 +1596,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     double frac = (bp && bp->mem_fraction > 0) ? bp->mem_fraction : 0.8;
     size_t per = batch_slot_bytes<T>(n, mp);
     CertWork &CW = cert_work(c);
-    CW.ensure(n, mp);
+    CW.ensure(n, mp, c.own);
     RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
     ll fit = (ll)((double)fr * frac / (double)per);
     int K = (bp && bp->slots > 0) ? bp->slots : (int)std::min<ll>(fit, 256);
@@ -1612,7 +1611,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     // tenth of what the states leave free (one at a time needs no more than a single solve's)
     const size_t cert_budget = std::min<size_t>((size_t)256 << 20, (fr - std::min(fr, (size_t)K * per)) / 10);
     const int KC = (int)std::max<size_t>(1, std::min<size_t>((size_t)K, cert_budget / CertWork::slot_bytes(n, mp)));
-    CW.ensure(n, mp, KC);
+    CW.ensure(n, mp, c.own, KC);
     // shared structure: observed positions, bits, per-menu masks, diagonal
     const DevProblem D = upload_problem(*pr, CW, st);
     BmCoef C = make_coef(n, par->beta, par->alpha, par->precond_p);
@@ -2013,7 +2012,7 @@ int push_ub64_host(Ctx &c, int n, int dtype, const void *x, ll mp, const uint32_
     cudaStream_t st = c.own;
     c.join_in();
     CertWork &CW = cert_work(c);
-    CW.ensure(n, mp);
+    CW.ensure(n, mp, c.own);
     const DevProblem D = upload_problem(pr, CW, st);
     setup_obs<double>(c, CW, nullptr, pr, D, st);
     Scratch &S = scratch(c);
@@ -2048,7 +2047,7 @@ int fw_lb64_host(Ctx &c, int n, ll mp, const uint32_t *menu, const int32_t *alt,
     cudaStream_t st = c.own;
     c.join_in();
     CertWork &CW = cert_work(c);
-    CW.ensure(n, mp);
+    CW.ensure(n, mp, c.own);
     const DevProblem D = upload_problem(pr, CW, st);
     // the y slab: scatter y at the observed positions through the xhat path (xhat := y)
     CW.y.ensure((size_t)mp * 8);
