@@ -262,14 +262,15 @@ static_assert((PE_R / 32) * PE_G == 32 && (PE_G & (PE_G - 1)) == 0, "32 warps; P
 // Layers whose 128-rank CTAs would not give every SM two of them run 32 ranks per CTA (8 warps).
 constexpr int PE_R_SMALL = 32;
 
-//
 // The sums w(x, D) do not depend on the layer before, only its values do: a layer's CTAs form their sums
 // from the pricer's lists and the call's scores (both complete before the sweep's first layer
 // started) while the layers before still run, and wait for them only then. The layers are chains of
 // dependent loads on a few hundred CTAs, so they overlap almost whole: a u24 sweep at n = 18 (0.5 % of the
-// menus) 403 -> 300 us.
+// menus) 403 -> 300 us. Held to 32 registers, so that an SM's 2,048 threads are all there: where a thread
+// reads its lists or tests rows the loads' latency is hidden by warps alone (n = 20, 0.3 % of the menus, u24:
+// 1,005 us at 48 registers, 878 at 32; n = 22, pairs, row tests, u16: 2,841 and 2,265).
 template <bool MASK, int PR>
-__global__ void __launch_bounds__(PR * PE_G) layer_eval_kernel(PricerArgs A, float *vals) {
+__global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kernel(PricerArgs A, float *vals) {
     pdl_launch_next();                                     // launched by launch_pdl
     static_assert(PR % 32 == 0 && (PR / 32) * PE_G <= 32, "at most 32 warps");
     __shared__ float pbest[PE_G][PR];
