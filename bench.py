@@ -84,7 +84,8 @@ def load_peaks():
 
 
 # the kernel sources whose digest a committed ncu summary must match for its DRAM figure to count
-KERNEL_SOURCES = {"prox": ("prox.cu", "prox.cuh"), "xform": ("xform.cuh",)}
+KERNEL_SOURCES = {"prox": ("prox.cu", "prox.cuh"), "xform": ("xform.cuh",),
+                  "dr_low": ("dr.cu", "dr.cuh")}
 
 
 def source_digest(kernel):

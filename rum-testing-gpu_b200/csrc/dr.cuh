@@ -20,9 +20,11 @@
 // alternative (2^(M-1) values for i < M, 2^M for i >= M and in the base mask); those runs are
 // exactly the low window's transforms, M - 1 bits for i < M and M bits for the others, and the high
 // window is the rest. Lattices beyond the two windows run middle passes on both streams.
-// Measured on one B200, an iteration at n = 13 / 16 / 18 / 20 / 22 in a replayed graph with its share of
-// the checks: 14.5 / 20.8 / 52.0 / 267 / 1,493 us, against 17.9 / 30.1 / 92 / 444 / 2,190 us for the
-// transform passes with the prox.
+// Measured on one B200, an iteration in a replayed graph: 10.3 / 14.6 / 44.0 / 249 / 1,319 us at n = 13 / 16 /
+// 18 / 20 / 22, where the transform passes with the prox took 17.9 / 30.1 / 92 / 444 / 2,190 us with their
+// share of the checks. What bounds it: latency of the two kernels to n = 16, the low kernel's dependent prox
+// steps at n = 18 (its slabs stay in L2), the high kernel's exchanges through shared memory at n = 20, and
+// memory from n = 21.
 #pragma once
 #include "xform.cuh"
 
@@ -44,8 +46,9 @@ struct DrArgs {
     const int *active;
 };
 
-// Smaller lattices are left to the one-pass transform and the lanes prox (n = 12: 12.0 us an iteration
-// against 13.9 here; n = 13: 17.9 against 14.5).
+// Smaller lattices are left to the one-pass transform and the lanes prox. Both sides with dependent launches
+// and their share of the checks: n = 12 12.0 us an iteration against 13.9 here, n = 13 17.9 against 14.5; since
+// then plain launches took the former to 9.6 and the latter to 11.9.
 constexpr int DR_MIN_N = 13;
 
 // One iteration's launches (n >= DR_MIN_N); last: also write u_out and t_out.

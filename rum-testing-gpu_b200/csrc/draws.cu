@@ -19,8 +19,8 @@
 // Layout: W row-major (B x R, float64); offered by menu and chose by row as CSR lists of
 // (respondent, count). A CTA takes DB draws: their weights side by side in shared memory, so that one
 // read of a list entry (from L2: what bounds the kernel) serves DB draws, and every menu's seen is summed
-// once and kept there for the menu's rows. 2,000 draws of 10,856 rows and 520 respondents (n = 16): a screen call takes 221 us
-// against 405 us with one draw per CTA and seen summed again for every row.
+// once and kept there for the menu's rows. 2,000 draws of 10,856 rows and 520 respondents (n = 16): a screen
+// call takes 218 us against 410 us with one draw per CTA and seen summed again for every row.
 #include <algorithm>
 #include <cmath>
 #include <memory>
