@@ -679,11 +679,11 @@ __global__ void mask_readout_kernel(int n, const float *V, const uint8_t *pred, 
 // the tile's low bits, L = lane + 32 j: bits 0-4 the lane, bits 5-7 the thread's register j). One
 // warp computes one tile; one launch covers the tiles whose high part H has popcount t, for
 // t = 0 .. n - 8, so every tile H ^ {x} a tile reads was written by the launch before. Per tile:
-//   w(x, D) for every x in D: one pass over x's rows for the whole tile. A row whose menu's high
-//     part is not a subset of H fails for all 256 masks (a warp-uniform skip); otherwise the lane
-//     test (menu bits 0-4 within the lane's) gives the lane's addend (the score or +0, which leaves
-//     a sum unchanged: a sum that starts at +0 is never -0) and a warp-uniform switch on the menu's
-//     bits 5-7 adds it to the registers j that contain them, in row order;
+//   w(x, D) for every x in D: one pass over x's rows for the whole tile (mt_rows). A row whose menu's
+//     high part is not a subset of H fails for all 256 masks (a bit of the warp's ballot); otherwise the
+//     lane test (menu bits 0-4 within the lane's) gives the lane's addend (the score or +0, which leaves
+//     a sum unchanged: a sum that starts at +0 is never -0) and the menu's bits 5-7 say which registers
+//     j contain them, in row order;
 //   high x in H: V[D \ {x}] is the same L of tile H ^ {x} (coalesced loads), merged at once;
 //   low x in L: V[D \ {x}] is a mask of the same tile, so the tile's values and w(x, D) go to
 //     shared memory and the low candidates are merged by popcount rounds of L (the masks of
@@ -721,9 +721,7 @@ __global__ void rows_kernel(ll mp, const ull *menus, const float *scores, const 
                         (int)(unsigned)((m >> 5) & 7ULL));
 }
 
-// Row records are read ROW_PF at a time ahead of their use; ROW_NONE pads the last batch (its high
-// part has every bit set, so no tile or group takes it: their high parts have at most 29 bits).
-constexpr int ROW_PF = 4;
+// A record no tile or group takes: its high part has every bit set, theirs at most 29.
 #define ROW_NONE make_int4(-1, 0, 0, 0)
 
 // Row records of the float64 max sweep's group form: {menu >> shift, menu & ymask, score low and
@@ -747,20 +745,47 @@ __device__ __forceinline__ void mt_merge(T &v, int &b, T c, int x) {
     }
 }
 
-// acc[j] += s for the registers j that contain mr (j's bits 5-7 of L; mr warp-uniform).
-__device__ __forceinline__ void mt_add(float (&acc)[MT_REGS], int mr, float s) {
-#define MT_A(j) acc[j] = __fadd_rn(acc[j], s)
-    switch (mr) {
-        case 0: MT_A(0); MT_A(1); MT_A(2); MT_A(3); MT_A(4); MT_A(5); MT_A(6); MT_A(7); break;
-        case 1: MT_A(1); MT_A(3); MT_A(5); MT_A(7); break;
-        case 2: MT_A(2); MT_A(3); MT_A(6); MT_A(7); break;
-        case 3: MT_A(3); MT_A(7); break;
-        case 4: MT_A(4); MT_A(5); MT_A(6); MT_A(7); break;
-        case 5: MT_A(5); MT_A(7); break;
-        case 6: MT_A(6); MT_A(7); break;
-        default: MT_A(7); break;
+// One alternative's row pass over a tile: acc[j] += score for the masks L = lane + 32 j whose subsets hold the
+// row's menu, in row order, from rows [lo, hi). The warp reads 32 records at a time, a lane each, and one
+// ballot drops the rows whose high part is not within H (nH = ~H); the others' low byte and score go round by
+// shuffle. Registers 2i and 2i + 1 are one packed accumulator (add.rn.f32x2 rounds each half as add.rn.f32):
+// a row is added to the pairs i that hold its bits 6-7, to the even register only without bit 5, and a lane
+// without its bits 0-4 adds +0. What bounds it is issue; a call
+// on mask storage with pairs as menus takes 3.14 ms at n = 26 and 12.5 ms at n = 28, against 4.45 and 18.0 with
+// four uniform loads and tests ahead, a switch on bits 5-7 and up to eight adds a row; 11,789 rows at n = 18
+// 0.62 against 1.64 ms.
+__device__ __forceinline__ void mt_add2(ull &acc, float even, float odd) {
+    asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%1, %2};\n\tadd.rn.f32x2 %0, %0, v;\n\t}" : "+l"(acc) : "f"(even), "f"(odd));
+}
+__device__ __forceinline__ void mt_rows(float (&acc)[MT_REGS], const int4 *rows, int lo, int hi, unsigned nH, int lane) {
+    static_assert(MT_REGS == 8, "pairs by bits 6-7, halves by bit 5");
+    const unsigned nlane = ~(unsigned)lane & 31u;
+    ull pair[MT_REGS / 2] = {0ULL, 0ULL, 0ULL, 0ULL};       // +0 twice
+    for (int i0 = lo; i0 < hi; i0 += 32) {                  // uniform per warp
+        int4 R = ROW_NONE;
+        if (i0 + lane < hi) R = __ldg(rows + i0 + lane);
+        const unsigned low = (unsigned)R.y | ((unsigned)R.w << 5);
+        unsigned todo = __ballot_sync(0xffffffffu, ((unsigned)R.x & nH) == 0u);
+        while (todo) {
+            const int b = __ffs((int)todo) - 1;
+            todo &= todo - 1u;
+            const unsigned m = __shfl_sync(0xffffffffu, low, b);
+            float s = __int_as_float(__shfl_sync(0xffffffffu, R.z, b));
+            if (m & nlane) s = 0.0f;
+            const float even = (m & 32u) ? 0.0f : s;
+            mt_add2(pair[3], even, s);
+            if (!(m & 64u)) mt_add2(pair[2], even, s);
+            if (!(m & 128u)) {
+                mt_add2(pair[1], even, s);
+                if (!(m & 64u)) mt_add2(pair[0], even, s);
+            }
+        }
     }
-#undef MT_A
+#pragma unroll
+    for (int i = 0; i < MT_REGS / 2; ++i) {
+        acc[2 * i] = __uint_as_float((unsigned)pair[i]);
+        acc[2 * i + 1] = __uint_as_float((unsigned)(pair[i] >> 32));
+    }
 }
 
 // The 256 low masks ordered by popcount (ascending masks within one popcount), and where each
@@ -810,7 +835,7 @@ __global__ void __launch_bounds__(32 * MT_WARPS) mask_tile_kernel(MaskTileArgs A
             --b;
         }
     }
-    const unsigned nH = ~H, nlane = ~(unsigned)lane;
+    const unsigned nH = ~H;
     const ull base = (ull)H << MT_LOW;
     float best[MT_REGS];
     int bx[MT_REGS];
@@ -829,20 +854,7 @@ __global__ void __launch_bounds__(32 * MT_WARPS) mask_tile_kernel(MaskTileArgs A
             for (int j = 0; j < MT_REGS; ++j) prev[j] = pv[32 * j];
         }
         float acc[MT_REGS];
-#pragma unroll
-        for (int j = 0; j < MT_REGS; ++j) acc[j] = 0.0f;
-        const int lo = (int)A.offsets[x], hi = (int)A.offsets[x + 1];
-        for (int i0 = lo; i0 < hi; i0 += ROW_PF) {
-            int4 R[ROW_PF];                                     // loaded ahead: the skips depend on them
-#pragma unroll
-            for (int u = 0; u < ROW_PF; ++u) R[u] = i0 + u < hi ? __ldg(A.rows + i0 + u) : ROW_NONE;
-#pragma unroll
-            for (int u = 0; u < ROW_PF; ++u) {
-                if ((unsigned)R[u].x & nH) continue;            // uniform: fails for the whole tile
-                const float s = ((unsigned)R[u].y & nlane) ? 0.0f : __int_as_float(R[u].z);
-                mt_add(acc, R[u].w, s);
-            }
-        }
+        mt_rows(acc, A.rows, (int)A.offsets[x], (int)A.offsets[x + 1], nH, lane);
         if (high) {
 #pragma unroll
             for (int j = 0; j < MT_REGS; ++j) mt_merge(best[j], bx[j], __fadd_rn(prev[j], acc[j]), x);
@@ -917,7 +929,7 @@ __global__ void __launch_bounds__(32 * MT_SPLIT) mask_tile_split_kernel(MaskTile
             --b;
         }
     }
-    const unsigned nH = ~H, nlane = ~(unsigned)lane;
+    const unsigned nH = ~H;
     const ull base = (ull)H << MT_LOW;
     float best[MT_REGS];
     int bx[MT_REGS];
@@ -936,20 +948,7 @@ __global__ void __launch_bounds__(32 * MT_SPLIT) mask_tile_split_kernel(MaskTile
             for (int j = 0; j < MT_REGS; ++j) prev[j] = pvp[32 * j];
         }
         float acc[MT_REGS];
-#pragma unroll
-        for (int j = 0; j < MT_REGS; ++j) acc[j] = 0.0f;
-        const int lo = (int)A.offsets[x], hi = (int)A.offsets[x + 1];
-        for (int i0 = lo; i0 < hi; i0 += ROW_PF) {
-            int4 R[ROW_PF];
-#pragma unroll
-            for (int u = 0; u < ROW_PF; ++u) R[u] = i0 + u < hi ? __ldg(A.rows + i0 + u) : ROW_NONE;
-#pragma unroll
-            for (int u = 0; u < ROW_PF; ++u) {
-                if ((unsigned)R[u].x & nH) continue;
-                const float sc = ((unsigned)R[u].y & nlane) ? 0.0f : __int_as_float(R[u].z);
-                mt_add(acc, R[u].w, sc);
-            }
-        }
+        mt_rows(acc, A.rows, (int)A.offsets[x], (int)A.offsets[x + 1], nH, lane);
         if (high) {
 #pragma unroll
             for (int j = 0; j < MT_REGS; ++j) mt_merge(best[j], bx[j], __fadd_rn(prev[j], acc[j]), x);

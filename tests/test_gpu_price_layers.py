@@ -45,3 +45,35 @@ def test_ranking_columns_at_word_edges(ctx):
             np.testing.assert_array_equal(got, np.asarray(O.ranking_column(n, menus, alts, rank)).astype(bool))
         cg.close()
         pr.close()
+
+
+@pytest.mark.parametrize("n", [9, 11, 22])
+def test_tile_row_pass_at_batch_edges(ctx, monkeypatch, n):
+    """The tile sweep's row pass reads 32 rows at a time: alternatives with 0, 1, 31, 32, 33, 64 and 65 rows,
+    few low bits and few high bits per menu, split tiles (n = 9, 11) and a warp per tile (n = 22), bit for bit
+    the oracle's sweep (n <= 11) or the layer kernels' (n = 22), also with scores of one sign and with zeros."""
+    rng = np.random.default_rng(n)
+    counts = [0, 1, 31, 32, 33, 64, 65]
+    menus, offsets = [], [0]
+    for x in range(n):
+        sets = set()
+        while len(sets) < counts[x % len(counts)]:
+            d = rng.random(n) < rng.choice([0.1, 0.3, 0.6])
+            d[x] = True
+            sets.add(int(sum(1 << int(i) for i in np.nonzero(d)[0])))
+        menus += sorted(sets)
+        offsets.append(len(menus))
+    menus, offsets = np.array(menus, np.uint64), np.array(offsets, np.int64)
+    pr = {}
+    for form in ("tile", "layer"):
+        monkeypatch.setenv("RUMB_MASK_FORM", form)
+        pr[form] = _lib.Pricer(ctx, n, menus, offsets, mode="mask")
+        monkeypatch.delenv("RUMB_MASK_FORM")
+    base = rng.standard_normal(menus.size).astype(np.float32)
+    for s in (base, -np.abs(base), np.where(rng.random(menus.size) < 0.5, np.float32(0), base)):
+        v, r, _ = pr["tile"].price(s)
+        want = O.price_mask(n, menus, s, offsets) if n <= 11 else pr["layer"].price(s)[:2]
+        assert v == want[0]
+        np.testing.assert_array_equal(r, want[1])
+    for p in pr.values():
+        p.close()
