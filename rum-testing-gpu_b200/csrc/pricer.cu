@@ -1028,7 +1028,7 @@ __global__ void sub_readout_kernel(int K, const float *V, const uint8_t *pred, S
 // stream_decode_kernel when the float32 copy fits) and candidates merge with the larger value
 // winning and, on equal values, the lower x (the row scan's x descending with `>=`): the layer is
 // the layer kernels' bit for bit, and stream_quant_kernel quantizes it as before.
-constexpr int SG_LOW = 10, SG_REGS = 8, SG_WARPS = 4, SG_PF = 4;   // SG_PF: rows read ahead
+constexpr int SG_LOW = 10, SG_REGS = 8, SG_WARPS = 4;
 constexpr int SG_MIN_N = SG_LOW + 2;
 
 struct StreamGroupArgs {
@@ -1040,6 +1040,27 @@ struct StreamGroupArgs {
     const double *vprev64;     // the float64 max sweep: previous and current layer
     double *vcur64;
 };
+
+// f(low part, score) for each of rows [lo, hi) whose high part lies within H (nH = ~H), in row order: the warp
+// reads 32 records at a time, a lane each, one ballot drops the others and the kept go round by shuffle
+// (u16 against four uniform loads and tests ahead: n = 22, pairs 1,248 and 1,499 us; n = 26 9.5 and 11.7 ms;
+// 11,789 rows at n = 18 9.0 and 14.8 ms; the float64 max sweep there 9.3 and 12.8 ms).
+template <class T, class F>
+__device__ __forceinline__ void sg_rows(const int4 *rows, int lo, int hi, unsigned nH, int lane, F f) {
+    for (int i0 = lo; i0 < hi; i0 += 32) {                  // uniform per warp
+        int4 R = ROW_NONE;
+        if (i0 + lane < hi) R = __ldg(rows + i0 + lane);
+        unsigned todo = __ballot_sync(0xffffffffu, ((unsigned)R.x & nH) == 0u);
+        while (todo) {
+            const int b = __ffs((int)todo) - 1;
+            todo &= todo - 1u;
+            const unsigned ml = (unsigned)__shfl_sync(0xffffffffu, R.y, b);
+            const int z = __shfl_sync(0xffffffffu, R.z, b);
+            if constexpr (sizeof(T) == 8) f(ml, __hiloint2double(__shfl_sync(0xffffffffu, R.w, b), z));
+            else f(ml, __int_as_float(z));
+        }
+    }
+}
 
 // One group's slots, NR registers per lane (NR * 32 >= the group's C(SG_LOW, l) slots).
 // T = float: the pricing sweep (values decoded from the previous layer, predecessors, lowest x on
@@ -1099,22 +1120,11 @@ __device__ __forceinline__ void sg_group(const PricerArgs &A, const StreamGroupA
                     accc[jc] = (T)0;
                 }
                 const int lo = (int)A.offsets[x], hi = (int)A.offsets[x + 1];
-                for (int i0 = lo; i0 < hi; i0 += SG_PF) {
-                    int4 R[SG_PF];
+                sg_rows<T>(G.rows, lo, hi, nH, lane, [&](unsigned ml, T sc) {
 #pragma unroll
-                    for (int u = 0; u < SG_PF; ++u) R[u] = i0 + u < hi ? __ldg(G.rows + i0 + u) : ROW_NONE;
-#pragma unroll
-                    for (int u = 0; u < SG_PF; ++u) {
-                        if ((unsigned)R[u].x & nH) continue;        // uniform: fails for the whole group
-                        const unsigned ml = (unsigned)R[u].y;
-                        T sc;
-                        if constexpr (sizeof(T) == 8) sc = __hiloint2double(R[u].w, R[u].z);
-                        else sc = __int_as_float(R[u].z);
-#pragma unroll
-                        for (int jc = 0; jc < NRC; ++jc)
-                            if (!(ml & nLc[jc])) accc[jc] = add_rn(accc[jc], sc);
-                    }
-                }
+                    for (int jc = 0; jc < NRC; ++jc)
+                        if (!(ml & nLc[jc])) accc[jc] = add_rn(accc[jc], sc);
+                });
 #pragma unroll
                 for (int jc = 0; jc < NRC; ++jc)
                     if (lane + 32 * jc < c9) cbuf[srk[Lc[jc]]] = add_rn(prevc[jc], accc[jc]);
@@ -1140,27 +1150,16 @@ __device__ __forceinline__ void sg_group(const PricerArgs &A, const StreamGroupA
 #pragma unroll
         for (int j = 0; j < NR; ++j) acc[j] = (T)0;
         const int lo = (int)A.offsets[x], hi = (int)A.offsets[x + 1];
-        for (int i0 = lo; i0 < hi; i0 += SG_PF) {
-            int4 R[SG_PF];
+        sg_rows<T>(G.rows, lo, hi, nH, lane, [&](unsigned ml, T sc) {
+            if (ml == 0u) {                                 // uniform: a menu within H fits every slot
 #pragma unroll
-            for (int u = 0; u < SG_PF; ++u) R[u] = i0 + u < hi ? __ldg(G.rows + i0 + u) : ROW_NONE;
+                for (int j = 0; j < NR; ++j) acc[j] = add_rn(acc[j], sc);
+            } else {
 #pragma unroll
-            for (int u = 0; u < SG_PF; ++u) {
-                if ((unsigned)R[u].x & nH) continue;            // uniform: fails for the whole group
-                const unsigned ml = (unsigned)R[u].y;
-                T sc;
-                if constexpr (sizeof(T) == 8) sc = __hiloint2double(R[u].w, R[u].z);
-                else sc = __int_as_float(R[u].z);
-                if (ml == 0u) {                                 // uniform: a menu within H fits every slot
-#pragma unroll
-                    for (int j = 0; j < NR; ++j) acc[j] = add_rn(acc[j], sc);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < NR; ++j)
-                        if (!(ml & nLj[j])) acc[j] = add_rn(acc[j], sc);
-                }
+                for (int j = 0; j < NR; ++j)
+                    if (!(ml & nLj[j])) acc[j] = add_rn(acc[j], sc);
             }
-        }
+        });
 #pragma unroll
         for (int j = 0; j < NR; ++j) {
             const int sl = lane + 32 * j;

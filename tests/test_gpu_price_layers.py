@@ -47,12 +47,8 @@ def test_ranking_columns_at_word_edges(ctx):
         pr.close()
 
 
-@pytest.mark.parametrize("n", [9, 11, 22])
-def test_tile_row_pass_at_batch_edges(ctx, monkeypatch, n):
-    """The tile sweep's row pass reads 32 rows at a time: alternatives with 0, 1, 31, 32, 33, 64 and 65 rows,
-    few low bits and few high bits per menu, split tiles (n = 9, 11) and a warp per tile (n = 22), bit for bit
-    the oracle's sweep (n <= 11) or the layer kernels' (n = 22), also with scores of one sign and with zeros."""
-    rng = np.random.default_rng(n)
+def _edge_menus(n, rng):
+    """Alternatives with 0, 1, 31, 32, 33, 64 and 65 rows in turn."""
     counts = [0, 1, 31, 32, 33, 64, 65]
     menus, offsets = [], [0]
     for x in range(n):
@@ -63,7 +59,16 @@ def test_tile_row_pass_at_batch_edges(ctx, monkeypatch, n):
             sets.add(int(sum(1 << int(i) for i in np.nonzero(d)[0])))
         menus += sorted(sets)
         offsets.append(len(menus))
-    menus, offsets = np.array(menus, np.uint64), np.array(offsets, np.int64)
+    return np.array(menus, np.uint64), np.array(offsets, np.int64)
+
+
+@pytest.mark.parametrize("n", [9, 11, 22])
+def test_tile_row_pass_at_batch_edges(ctx, monkeypatch, n):
+    """The tile sweep's row pass reads 32 rows at a time: alternatives with 0, 1, 31, 32, 33, 64 and 65 rows,
+    few low bits and few high bits per menu, split tiles (n = 9, 11) and a warp per tile (n = 22), bit for bit
+    the oracle's sweep (n <= 11) or the layer kernels' (n = 22), also with scores of one sign and with zeros."""
+    rng = np.random.default_rng(n)
+    menus, offsets = _edge_menus(n, rng)
     pr = {}
     for form in ("tile", "layer"):
         monkeypatch.setenv("RUMB_MASK_FORM", form)
@@ -77,3 +82,19 @@ def test_tile_row_pass_at_batch_edges(ctx, monkeypatch, n):
         np.testing.assert_array_equal(r, want[1])
     for p in pr.values():
         p.close()
+
+
+@pytest.mark.parametrize("mode", ["u16", "f32"])
+def test_group_row_pass_at_batch_edges(ctx, monkeypatch, mode):
+    """The group sweep's row pass (32 rows at a time) on the same menus at n = 13: the layer kernels' value and
+    ranking, and their float64 maximum, bit for bit."""
+    n, rng, got = 13, np.random.default_rng(13), {}
+    menus, offsets = _edge_menus(n, rng)
+    s = rng.standard_normal(menus.size).astype(np.float32)
+    for form in ("group", "layer"):
+        monkeypatch.setenv("RUMB_STREAM_FORM", form)
+        pr = _lib.Pricer(ctx, n, menus, offsets, mode=mode, stream=mode == "f32")
+        v, r, _ = pr.price(s)
+        got[form] = (v, r.tolist(), pr.max64(s.astype(np.float64)))
+        pr.close()
+    assert got["group"] == got["layer"]
