@@ -459,9 +459,9 @@ struct BmCoef {
     // A Q divided by q00; the scales q00^(n-1) of Q and of Q^T move into the diagonal
     double Qu[4], AQu[4];
     std::vector<double> diag;   // by popcount: entries 0..nb as is, 32..32+nb times q00^(2 nb)
-    int lo_bits = 12;           // transform window split (tuned)
-    int prox_form = PROX_TILE;  // prox kernel form (tuned)
-    int fuse = 1;               // two windows: P4 carries the next A' (three passes an iteration; tuned)
+    int lo_bits = 12;           // the transforms' low window
+    int prox_form = PROX_TILE;  // prox kernel form
+    int fuse = 1;               // two windows: P4 carries the next A' (three passes an iteration)
     bool dr = false;            // the two-kernel iteration (dr.cuh)
 };
 
@@ -741,12 +741,6 @@ static void enqueue_cold_start(BmWork<T> &W, const BmCoef &C, int n, cudaStream_
     for (DevBuf *b : {&W.s, &W.y, &W.z}) RUMB_CUDA(cudaMemsetAsync(b->ptr, 0, (size_t)m2 * sizeof(T), st));
 }
 
-// The iteration's autotuner: times a few iterations of each candidate on the workspace and keeps
-// the fastest, one knob at a time -- the transform passes' low-window size (10, 11 or 12 bits;
-// it sets the high-window split), then the prox kernel's form (the shared-memory tile, or 2, 4 or
-// 8 lanes per menu), then with two windows the fused three-pass sequence against four passes.
-// Cached per context, n and dtype; the state is reset by the caller. The environment variables
-// RUMB_PROX_FORM (0 tile, 1..3 lanes 2/4/8) and RUMB_FUSE (0 / 1) pin those knobs.
 static int forced_knob(const char *name, int count) {
     const char *e = getenv(name);
     if (!e || !*e) return -1;
@@ -759,88 +753,32 @@ template <class T>
 static bool takes_dr(int n) {
     return sizeof(T) == 8 && n >= DR_MIN_N && forced_knob("RUMB_PROX_FORM", PROX_FORMS) < 0 && forced_knob("RUMB_FUSE", 2) < 0;
 }
-static void apply_forced(BmCoef &C) {
+// The sequence of the iteration at n alternatives in state type T: the transforms' low window, the prox kernel's
+// form and, with two windows, fused passes. A rule, not a timing on the spot: windows and forms add in different
+// orders, and a float32 state's fit moves by 0.1-1 % with them, so every solve, batch and bm_iterate call takes the
+// same. The orders are the window's, and two of a menu's members: tile, tau and the lanes forms give the same bits,
+// tau2 and pair others. Within an order the fastest form is taken, us an iteration in a replayed graph, float32:
+//   n = 8 lanes8 3.9, lanes4 4.4, tau 6.2; n = 13 8.7 / 9.6 / 11.9; n = 14 10.2 / 10.9 / 13.3; n = 15 13.5 / 12.7 /
+//   14.9; n = 16 20.7 / 19.0 / 18.6; n = 18 79.7 / 66.4 / 51.8; n = 20 tau2 227.5, pair 240; n = 22 1,252 / 1,328;
+//   n = 23 tile 3,160, tau 3,019; n = 25 13,370 / 12,800
+// and float64 (up to DR_MIN_N): n = 8 lanes8 4.1, lanes4 4.6, pair 6.1; n = 12 7.9 / 8.3 / 10.2. float64 from there on
+// comes here with a pinned knob only: RUMB_PROX_FORM (the forms of prox.cuh) and RUMB_FUSE (0 / 1) pin those two.
+template <class T>
+static void set_sequence(BmCoef &C, int n) {
+    C.dr = takes_dr<T>(n);
+    C.fuse = 1;
+    C.lo_bits = 12;
+    if (sizeof(T) == 4) {
+        if ((n >= 14 && n <= 16) || n == 22) C.lo_bits = 10;
+        C.prox_form = n <= 14 ? PROX_LANES8 : n == 15 ? PROX_LANES4 : n >= 19 && n <= 22 ? PROX_TAU2 : PROX_TAU;
+    } else {
+        if (n >= 13 && n <= 19) C.lo_bits = n <= 16 ? 10 : 11;
+        C.prox_form = n <= 14 ? PROX_LANES8 : n <= 16 ? PROX_LANES4 : n <= 22 ? PROX_PAIR : PROX_TILE;
+    }
     int f = forced_knob("RUMB_PROX_FORM", PROX_FORMS);
     if (f >= 0) C.prox_form = f;
     f = forced_knob("RUMB_FUSE", 2);
     if (f >= 0) C.fuse = f;
-}
-
-template <class T>
-static void tune_iteration(Ctx &c, BmWork<T> &W, BmCoef &C, int n, cudaStream_t st) {
-    C.dr = takes_dr<T>(n);
-    if (C.dr) return;                                        // nothing to tune
-    auto key = std::make_pair(n, (int)sizeof(T));
-    auto it = c.tuned.find(key);
-    if (it == c.tuned.end()) {
-        BmCoef K = C;
-        enqueue_cold_start<T>(W, C, n, st);                  // a state to time on
-        cudaEvent_t a, b;
-        RUMB_CUDA(cudaEventCreate(&a));
-        RUMB_CUDA(cudaEventCreate(&b));
-        auto time_it = [&]() -> float {
-            enqueue_iterations<T>(W, K, n, st, 2);
-            RUMB_CUDA(cudaEventRecord(a, st));
-            enqueue_iterations<T>(W, K, n, st, 6);
-            RUMB_CUDA(cudaEventRecord(b, st));
-            RUMB_CUDA(cudaEventSynchronize(b));
-            float ms = 0.f;
-            RUMB_CUDA(cudaEventElapsedTime(&ms, a, b));
-            return ms;
-        };
-        int best_lo = 12, best_form = n <= PROX_LANES_MAX_N ? PROX_LANES4 : PROX_TILE, best_fuse = 1;
-        if (n >= PT_M + 1) {
-            K.prox_form = best_form;
-            K.fuse = best_fuse;
-            if (n - 1 > 10) {
-                float best_ms = 1e30f;
-                for (int lb : {10, 11, 12}) {
-                    if (lb > n - 1) continue;
-                    K.lo_bits = lb;
-                    float ms = time_it();
-                    if (ms < best_ms) { best_ms = ms; best_lo = lb; }
-                }
-            }
-            K.lo_bits = best_lo;
-            if (n <= PROX_LANES_MAX_N) {
-                float best_ms = 1e30f;
-                for (int f = 0; f < PROX_FORMS; ++f) {
-                    K.prox_form = f;
-                    float ms = time_it();
-                    if (ms < best_ms) { best_ms = ms; best_form = f; }
-                }
-            }
-            K.prox_form = best_form;
-            if (xf_plan(n - 1, best_lo).size() == 2) {
-                float best_ms = 1e30f;
-                for (int f = 0; f < 2; ++f) {
-                    K.fuse = f;
-                    float ms = time_it();
-                    if (ms < best_ms) { best_ms = ms; best_fuse = f; }
-                }
-            }
-        }
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
-        it = c.tuned.emplace(key, std::array<int, 3>{best_lo, best_form, best_fuse}).first;
-    }
-    C.lo_bits = it->second[0];
-    C.prox_form = it->second[1];
-    C.fuse = it->second[2];
-    apply_forced(C);
-}
-
-// The tuned schedule of (n, dtype) when it is known, else the defaults.
-template <class T>
-static void tuned_or_default(Ctx &c, BmCoef &C, int n) {
-    C.dr = takes_dr<T>(n);
-    auto it = c.tuned.find(std::make_pair(n, (int)sizeof(T)));
-    if (it != c.tuned.end()) {
-        C.lo_bits = it->second[0];
-        C.prox_form = it->second[1];
-        C.fuse = it->second[2];
-    }
-    apply_forced(C);
 }
 
 // ----------------------------------------------------------------- problem upload
@@ -1291,11 +1229,10 @@ int bm_solve(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, const
     std::vector<float> d32(C.diag.begin(), C.diag.end());
     if (W32) RUMB_CUDA(cudaMemcpyAsync(W32->diag.ptr, d32.data(), d32.size() * 4, cudaMemcpyHostToDevice, st));
     if (W64) RUMB_CUDA(cudaMemcpyAsync(W64->diag.ptr, C.diag.data(), C.diag.size() * 8, cudaMemcpyHostToDevice, st));
-    // transform split (tuned once per context, n and dtype), then the initial state
     BmCoef C64 = C;
-    if (W32) tune_iteration<float>(c, *W32, C, n, st);
-    if (W64) tune_iteration<double>(c, *W64, C64, n, st);
-    if (!W32) C = C64;
+    set_sequence<double>(C64, n);
+    if (W32) set_sequence<float>(C, n);
+    else C = C64;
     if (use32) {
         if (warm) copy_state_in<float>(*W32, *warm, m2, st);
         else enqueue_cold_start<float>(*W32, C, n, st);
@@ -1382,7 +1319,7 @@ int bm_iterate(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, voi
         std::vector<T> dg(C.diag.begin(), C.diag.end());
         RUMB_CUDA(cudaMemcpyAsync(W.diag.ptr, dg.data(), dg.size() * sizeof(T), cudaMemcpyHostToDevice, st));
         size_t sb = (size_t)m2 * sizeof(T);
-        tuned_or_default<T>(c, C, n);
+        set_sequence<T>(C, n);
         if (cold) {
             enqueue_cold_start<T>(W, C, n, st);
         } else {
@@ -1438,7 +1375,7 @@ int bm_profile(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_params *par, int
         RUMB_CUDA(cudaMemsetAsync(W.err.ptr, 0, 16, st));
         std::vector<T> dg(C.diag.begin(), C.diag.end());
         RUMB_CUDA(cudaMemcpyAsync(W.diag.ptr, dg.data(), dg.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        tune_iteration<T>(c, W, C, n, st);
+        set_sequence<T>(C, n);
         enqueue_cold_start<T>(W, C, n, st);
         enqueue_begin<T>(iter_ptrs<T>(W), C, n, st);
         enqueue_iterations<T>(W, C, n, st, std::max(warmup, 3));      // warm-up
@@ -1642,8 +1579,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     I.slots = K;
     I.bstride = m2;
     I.active = W.active.template as<int>();
-    // the schedule tuned on a single-draw workspace, when known
-    tuned_or_default<T>(c, C, n);
+    set_sequence<T>(C, n);
     // the draws' rows, uploaded once; kept with the workspace up to 64 MB
     const size_t row_bytes = (size_t)B * (size_t)mp * 8;
     DevBuf own_p, own_y;

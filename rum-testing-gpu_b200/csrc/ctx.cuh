@@ -1,7 +1,6 @@
 // The library context: one device, one stream, cached lattice tables and workspaces.
 #pragma once
 #include <atomic>
-#include <array>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -33,9 +32,6 @@ struct Ctx {
     // they launch on, so that they go first
     std::unique_ptr<BmWorkBase> graphs64, graphs32, batch_graphs64, batch_graphs32;
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;   // a call's device time (made on first use)
-    // the iteration's tuned schedule per (n, state bytes): transform low-window size, prox form,
-    // fused passes (0 / 1)
-    std::map<std::pair<int, int>, std::array<int, 3>> tuned;
     // overlapped checks: a second stream and its two events; a check's pinned result words (made on first use)
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_snap = nullptr, ev_done = nullptr;

@@ -110,7 +110,7 @@ __device__ __forceinline__ ll pt_rstart(uint32_t base, int i, ll Nloc) {
 // each menu's members (the menu's threshold kept in shared memory, the projection and the write-back
 // done element by element; x, x2, z staged, or the relaxed point and z with a support bit); or G
 // lanes per menu reading the slab straight into registers
-// (n <= PROX_LANES_MAX_N). Picked per GPU, n and dtype by timing (the iteration's autotuner).
+// (n <= PROX_LANES_MAX_N). Picked by n and dtype (set_sequence, csrc/bm.cu).
 constexpr int PROX_TILE = 0, PROX_LANES2 = 1, PROX_LANES4 = 2, PROX_LANES8 = 3, PROX_TAU = 4, PROX_TAU2 = 5,
               PROX_PAIR = 6, PROX_FORMS = 7;
 constexpr int PROX_LANES_MAX_N = 22;

@@ -360,8 +360,8 @@ struct XfShape {
 };
 
 // Window split of nb rest bits: a low pass (s0 = 0) of up to lo_bits (<= 12) bits, then high
-// passes of up to 7 bits. Returns (L, RB, WB) per pass with RB >= WB, RB <= 4. The split is a
-// tuning knob (rumb picks lo_bits per GPU, n and dtype by timing the candidates).
+// passes of up to 7 bits. Returns (L, RB, WB) per pass with RB >= WB, RB <= 4. The iteration's
+// lo_bits follow from n and the dtype (set_sequence, csrc/bm.cu).
 inline std::vector<XfShape> xf_plan(int nb, int lo_bits = 12) {
     std::vector<XfShape> plan;
     if (lo_bits > 12) lo_bits = 12;
