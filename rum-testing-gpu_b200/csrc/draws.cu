@@ -20,7 +20,8 @@
 // (respondent, count). A CTA takes DB draws: their weights side by side in shared memory, so that one
 // read of a list entry (from L2: what bounds the kernel) serves DB draws, and every menu's seen is summed
 // once and kept there for the menu's rows. 2,000 draws of 10,856 rows and 520 respondents (n = 16): a screen
-// call takes 218 us against 410 us with one draw per CTA and seen summed again for every row.
+// call takes 218 us against 410 us with one draw per CTA and seen summed again for every row, the form that is left
+// where keeping it costs more (draw_keeps_seen).
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -48,9 +49,9 @@ struct DrawArgs {
 };
 
 // rows: count x M output (perturbed with scale when perturbed = 1, else the raw shares), or null;
-// dev / ub: per draw ||p_b - p_hat|| and ||perturb(p_b) - fit|| (ub needs fit), or null. CACHED: seen by menu in
-// shared memory (n_menus * DB values after the weights); else summed for every row.
-template <int DB, bool CACHED>
+// dev / ub: per draw ||p_b - p_hat|| and ||perturb(p_b) - fit|| (ub needs fit), or null. Seen by menu in shared
+// memory (n_menus * DB values after the weights).
+template <int DB>
 __global__ void __launch_bounds__(DR_THREADS) draw_rows_kernel(DrawArgs A, int n_menus, const ll *idx, ll count,
                                                                int perturbed, double scale, const double *fit,
                                                                double *rows, double *dev, double *ub) {
@@ -76,15 +77,13 @@ __global__ void __launch_bounds__(DR_THREADS) draw_rows_kernel(DrawArgs A, int n
         }
     };
     double *sseen = sw + (size_t)A.R * DB;
-    if (CACHED) {
-        for (int u = threadIdx.x; u < n_menus; u += blockDim.x) {
-            double v[DB];
-            list_sum(A.oresp, A.ocnt, A.optr[u], A.optr[u + 1], v);
+    for (int u = threadIdx.x; u < n_menus; u += blockDim.x) {
+        double v[DB];
+        list_sum(A.oresp, A.ocnt, A.optr[u], A.optr[u + 1], v);
 #pragma unroll
-            for (int q = 0; q < DB; ++q) sseen[u * DB + q] = v[q];
-        }
-        __syncthreads();
+        for (int q = 0; q < DB; ++q) sseen[u * DB + q] = v[q];
     }
+    __syncthreads();
     double sd[DB], su[DB];
 #pragma unroll
     for (int q = 0; q < DB; ++q) sd[q] = su[q] = 0.0;
@@ -93,12 +92,8 @@ __global__ void __launch_bounds__(DR_THREADS) draw_rows_kernel(DrawArgs A, int n
         const double ph = A.p_hat[j], fj = fit ? fit[j] : 0.0;
         double seen[DB], chose[DB];
         list_sum(A.cresp, A.ccnt, A.cptr[j], A.cptr[j + 1], chose);
-        if (CACHED) {
 #pragma unroll
-            for (int q = 0; q < DB; ++q) seen[q] = sseen[u * DB + q];
-        } else {
-            list_sum(A.oresp, A.ocnt, A.optr[u], A.optr[u + 1], seen);
-        }
+        for (int q = 0; q < DB; ++q) seen[q] = sseen[u * DB + q];
 #pragma unroll
         for (int q = 0; q < DB; ++q) {
             const double pb = seen[q] <= 0.0 ? ph : __ddiv_rn(chose[q], seen[q]);
@@ -138,9 +133,59 @@ __global__ void __launch_bounds__(DR_THREADS) draw_rows_kernel(DrawArgs A, int n
     }
 }
 
+// The same with one draw a CTA and seen summed again for every row.
+__global__ void __launch_bounds__(DR_THREADS) draw_rows_again_kernel(DrawArgs A, const ll *idx, int perturbed,
+                                                                     double scale, const double *fit, double *rows,
+                                                                     double *dev, double *ub) {
+    extern __shared__ double sw[];
+    __shared__ double red_d[DR_THREADS / 32], red_u[DR_THREADS / 32];
+    const ll b = idx ? idx[blockIdx.x] : (ll)blockIdx.x;
+    const double *wrow = A.W + b * (ll)A.R;
+    for (int r = threadIdx.x; r < A.R; r += blockDim.x) sw[r] = wrow[r];
+    __syncthreads();
+    double sd = 0.0, su = 0.0;
+    double *out = rows ? rows + (ll)blockIdx.x * A.M : nullptr;
+    for (ll j = threadIdx.x; j < A.M; j += blockDim.x) {
+        const int u = A.row_menu[j];
+        double seen = 0.0, chose = 0.0;
+        for (ll k = A.optr[u]; k < A.optr[u + 1]; ++k) seen = __dadd_rn(seen, __dmul_rn(sw[A.oresp[k]], A.ocnt[k]));
+        for (ll k = A.cptr[j]; k < A.cptr[j + 1]; ++k) chose = __dadd_rn(chose, __dmul_rn(sw[A.cresp[k]], A.ccnt[k]));
+        const double ph = A.p_hat[j];
+        const double pb = seen <= 0.0 ? ph : __ddiv_rn(chose, seen);
+        const double P = __dadd_rn(ph, __dmul_rn(scale, __dsub_rn(pb, ph)));
+        if (out) out[j] = perturbed ? P : pb;
+        const double d = __dsub_rn(pb, ph);
+        sd = __dadd_rn(sd, __dmul_rn(d, d));
+        if (fit) {
+            const double e = __dsub_rn(P, fit[j]);
+            su = __dadd_rn(su, __dmul_rn(e, e));
+        }
+    }
+    if (!dev && !ub) return;
+    for (int o = 16; o > 0; o >>= 1) {
+        sd += __shfl_xor_sync(0xffffffffu, sd, o);
+        su += __shfl_xor_sync(0xffffffffu, su, o);
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        red_d[w] = sd;
+        red_u[w] = su;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double td = 0.0, tu = 0.0;
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+            td += red_d[i];
+            tu += red_u[i];
+        }
+        if (dev) dev[blockIdx.x] = sqrt(td);
+        if (ub) ub[blockIdx.x] = sqrt(tu);
+    }
+}
+
 struct Draws {
     Ctx *c = nullptr;
-    ll B = 0, M = 0;
+    ll B = 0, M = 0, entries = 0;             // entries: of the offered lists
     int R = 0, n_menus = 0;
     DevBuf W, optr, oresp, ocnt, cptr, cresp, ccnt, row_menu, p_hat;
     DevBuf fit, idx, rows, dev, ub;
@@ -179,6 +224,7 @@ Draws *draws_create(Ctx &c, ll B, int R, ll M, int n_menus, const double *W, con
     D->R = R;
     D->M = M;
     D->n_menus = n_menus;
+    D->entries = optr[n_menus];
     cudaStream_t st = c.own;
     upload(D->W, W, (size_t)B * R, st);
     upload(D->optr, optr, (size_t)n_menus + 1, st);
@@ -214,27 +260,58 @@ static DrawArgs args_of(const Draws &D) {
 }
 
 constexpr size_t DRAW_SMEM = 200 * 1024;
-template <int DB, bool CACHED>
+template <int DB>
 static void launch_form(const Draws &D, ll count, const ll *idx, int perturbed, double scale, const double *fit, double *rows,
                         double *dev, double *ub) {
     static std::atomic<unsigned long long> optin{0};
-    const size_t smem = ((size_t)D.R + (CACHED ? (size_t)D.n_menus : 0)) * DB * sizeof(double);
-    smem_optin(draw_rows_kernel<DB, CACHED>, (int)DRAW_SMEM, optin);
-    draw_rows_kernel<DB, CACHED><<<(unsigned)((count + DB - 1) / DB), DR_THREADS, smem, D.c->own>>>(
+    const size_t smem = ((size_t)D.R + (size_t)D.n_menus) * DB * sizeof(double);
+    smem_optin(draw_rows_kernel<DB>, (int)DRAW_SMEM, optin);
+    draw_rows_kernel<DB><<<(unsigned)((count + DB - 1) / DB), DR_THREADS, smem, D.c->own>>>(
         args_of(D), D.n_menus, idx, count, perturbed, scale, fit, rows, dev, ub);
     RUMB_LAUNCH("draw_rows_kernel");
 }
 
-// Four draws a CTA while three such CTAs fit an SM, two while two do, as long as that leaves two CTAs per SM;
-// seen by menu wherever one draw's fits (28,000 menus and more sum it per row, as every size did before).
+static void launch_again(const Draws &D, ll count, const ll *idx, int perturbed, double scale, const double *fit, double *rows,
+                         double *dev, double *ub) {
+    static std::atomic<unsigned long long> optin{0};
+    smem_optin(draw_rows_again_kernel, (int)DRAW_SMEM, optin);
+    draw_rows_again_kernel<<<(unsigned)count, DR_THREADS, (size_t)D.R * sizeof(double), D.c->own>>>(
+        args_of(D), idx, perturbed, scale, fit, rows, dev, ub);
+    RUMB_LAUNCH("draw_rows_again_kernel");
+}
+
+// CTAs of `smem` dynamic bytes that an SM holds (227 KB, a kilobyte of it reserved per CTA; 2,048 threads).
+static int draw_ctas(size_t smem) {
+    return (int)std::min<size_t>(2048 / DR_THREADS, 227 * 1024 / (smem + 1300));
+}
+
+// Whether a draw of its own CTA keeps seen by menu: where the menus have four rows or more (with two a menu's list is
+// read about as often and by fewer threads: R 7,000, U 300 menus, B 600 draws 1,357 us a screen against 1,197) and it
+// does not cost more than it saves in CTAs of an SM or in L1 for the lists' reads. Kept / summed again, us a screen
+// (R respondents of 20 offers, five rows a menu): R 520, U 6,000, B 600 226 / 283; U 10,000, B 2,600 (two CTAs for
+// four) 1,112 / 1,256, but R 2,500, B 300 (a second wave for the last draws) 397 / 368; one CTA for four, R 1,000,
+// U 20,000, B 2,600 3,748 / 2,440, but few draws (B 100) 290 / 375; one for two, R 12,000, U 3,000 857 / 1,202; with
+// 140,000 entries and L1 left 28 KB (R 7,000, U 6,000) 777 / 659, 92 KB (U 3,000) 536 / 720; above 160 KB (R 20,000,
+// U 5,000, B 500) 4,106 / 2,117.
+static bool draw_keeps_seen(const Draws &D, ll count) {
+    const size_t r = (size_t)D.R * sizeof(double), one = r + (size_t)D.n_menus * sizeof(double);
+    const int sms = num_sms(D.c->device), with = draw_ctas(one), without = draw_ctas(r);
+    if (D.M < 4 * (ll)D.n_menus || one > DRAW_SMEM || (one > 160 * 1024 && without < 2)) return false;
+    if (count <= sms || with == without) return true;
+    if (with < 2) return without <= 2 && one <= 160 * 1024;
+    if (with == 2 && count > 2 * sms && count < 4 * sms) return false;
+    return D.entries <= 100000 || with * one <= 165 * 1024;
+}
+
+// Four draws a CTA while three such CTAs fit an SM, two while two do, as long as that leaves two CTAs per SM.
 static void launch(const Draws &D, ll count, const ll *idx, int perturbed, double scale, const double *fit,
                    double *rows, double *dev, double *ub) {
     const size_t one = ((size_t)D.R + (size_t)D.n_menus) * sizeof(double);
     const ll spread = 2 * num_sms(D.c->device);
-    if (one > DRAW_SMEM) launch_form<1, false>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
-    else if (4 * one <= 72 * 1024 && count >= 4 * spread) launch_form<4, true>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
-    else if (2 * one <= 108 * 1024 && count >= 2 * spread) launch_form<2, true>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
-    else launch_form<1, true>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
+    if (4 * one <= 72 * 1024 && count >= 4 * spread) launch_form<4>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
+    else if (2 * one <= 108 * 1024 && count >= 2 * spread) launch_form<2>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
+    else if (draw_keeps_seen(D, count)) launch_form<1>(D, count, idx, perturbed, scale, fit, rows, dev, ub);
+    else launch_again(D, count, idx, perturbed, scale, fit, rows, dev, ub);
 }
 
 void draws_rows(Draws *D, const int64_t *idx, ll count, int perturbed, double scale, double *out) {
