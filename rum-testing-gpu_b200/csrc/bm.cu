@@ -669,11 +669,15 @@ static void enqueue_iterations_ptrs(const IterPtrs<T> &I, const BmCoef &C, int n
             return;
         }
     }
-    // From n = 11 they go out in plain stream order: a CTA launched ahead waits on its SM beside the kernel
-    // before. us an iteration ahead / plain: float32 n = 11 7.3 / 7.0, n = 13 10.6 / 10.4, n = 15 17.5 / 14.5, n = 16
-    // 23.9 / 20.9, n = 17 31.1 / 29.3, n = 18 55.4 / 55.6, n = 20 236 / 233, n = 22 1,287 / 1,227, float64 n = 12
-    // 10.5 / 9.6; up to n = 10 launching ahead is even or the faster side (float64 n = 8 5.08 / 5.32).
-    PlainOrder order(n >= 11);
+    // Captured into a graph they go out in plain stream order from n = 11: a CTA launched ahead waits on its SM beside
+    // the kernel before. us an iteration ahead / plain in a replayed graph: float32 n = 11 5.9 / 5.7, n = 12 6.8 / 6.5,
+    // n = 14 12.0 / 10.2, n = 16 24.9 / 18.6, n = 18 51.9 / 51.8, n = 20 227.1 / 227.5, n = 22 1,350 / 1,252, float64
+    // n = 12 9.2 / 7.9; up to n = 10 launching ahead is even or the faster side (float64 n = 8 5.08 / 5.32). Launched one
+    // by one they wait for the host, and going ahead hides that to n = 21: float32 n = 11 6.9 / 8.3, n = 14 13.2 / 18.5,
+    // n = 18 52.8 / 60.5, n = 20 227.2 / 235.5, n = 22 1,366 / 1,295.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    RUMB_CUDA(cudaStreamIsCapturing(st, &cs));
+    PlainOrder order(n >= (cs == cudaStreamCaptureStatusActive ? 11 : 22));
     for (int i = 0; i < count; ++i) enqueue_iteration_ptrs<T>(I, C, n, st, i, count);
 }
 
@@ -759,8 +763,8 @@ static bool takes_dr(int n) {
 // same. The orders are the window's, and two of a menu's members: tile, tau and the lanes forms give the same bits,
 // tau2 and pair others. Within an order the fastest form is taken, us an iteration in a replayed graph, float32:
 //   n = 8 lanes8 3.9, lanes4 4.4, tau 6.2; n = 13 8.7 / 9.6 / 11.9; n = 14 10.2 / 10.9 / 13.3; n = 15 13.5 / 12.7 /
-//   14.9; n = 16 20.7 / 19.0 / 18.6; n = 18 79.7 / 66.4 / 51.8; n = 20 tau2 227.5, pair 240; n = 22 1,252 / 1,328;
-//   n = 23 tile 3,160, tau 3,019; n = 25 13,370 / 12,800
+//   14.9; n = 16 20.7 / 19.0 / 18.6 (launched one by one 24.9 / 23.3 / 24.6); n = 18 79.7 / 66.4 / 51.8;
+//   n = 20 tau2 227.5, pair 240; n = 22 1,252 / 1,328; n = 23 tile 3,160, tau 3,019; n = 25 13,370 / 12,800
 // and float64 (up to DR_MIN_N): n = 8 lanes8 4.1, lanes4 4.6, pair 6.1; n = 12 7.9 / 8.3 / 10.2. float64 from there on
 // comes here with a pinned knob only: RUMB_PROX_FORM (the forms of prox.cuh) and RUMB_FUSE (0 / 1) pin those two.
 template <class T>
@@ -770,7 +774,7 @@ static void set_sequence(BmCoef &C, int n) {
     C.lo_bits = 12;
     if (sizeof(T) == 4) {
         if ((n >= 14 && n <= 16) || n == 22) C.lo_bits = 10;
-        C.prox_form = n <= 14 ? PROX_LANES8 : n == 15 ? PROX_LANES4 : n >= 19 && n <= 22 ? PROX_TAU2 : PROX_TAU;
+        C.prox_form = n <= 14 ? PROX_LANES8 : n <= 16 ? PROX_LANES4 : n >= 19 && n <= 22 ? PROX_TAU2 : PROX_TAU;
     } else {
         if (n >= 13 && n <= 19) C.lo_bits = n <= 16 ? 10 : 11;
         C.prox_form = n <= 14 ? PROX_LANES8 : n <= 16 ? PROX_LANES4 : n <= 22 ? PROX_PAIR : PROX_TILE;
