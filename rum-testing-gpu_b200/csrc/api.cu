@@ -41,7 +41,8 @@ using rumb::Error;
 
 #define NEED_CTX(ctx)                                                  \
     if (!(ctx)) rumb::fail(RUMB_E_INVAL, "context is NULL");           \
-    rumb::DeviceGuard _dg((ctx)->c.device)
+    rumb::DeviceGuard _dg((ctx)->c.device);                            \
+    rumb::SpareGuard _sg(&(ctx)->c)
 
 extern "C" {
 
@@ -132,7 +133,7 @@ int rumb_mem_info(rumb_ctx *ctx, size_t *free_bytes, size_t *total_bytes) {
     NEED_CTX(ctx);
     size_t f = 0, t = 0;
     RUMB_CUDA(cudaMemGetInfo(&f, &t));
-    if (free_bytes) *free_bytes = f;
+    if (free_bytes) *free_bytes = f + ctx->c.bytes();      // with what a call of this context can have back
     if (total_bytes) *total_bytes = t;
     return RUMB_OK;
     RUMB_API_END
@@ -437,7 +438,8 @@ struct rumb_mlp {
 
 #define NEED_MLP(h)                                                    \
     if (!(h) || !(h)->m) rumb::fail(RUMB_E_INVAL, "mlp is NULL");      \
-    rumb::DeviceGuard _dg((h)->ctx->c.device)
+    rumb::DeviceGuard _dg((h)->ctx->c.device);                         \
+    rumb::SpareGuard _sg(&(h)->ctx->c)
 
 int rumb_gemm_bf16(rumb_ctx *ctx, int M, int N, int K, const uint16_t *A, const uint16_t *B, float *C) {
     RUMB_API_BEGIN

@@ -299,6 +299,13 @@ struct CertWork : public BmWorkBase {
     static size_t slot_bytes(int n, ll mp) {
         return 2 * 8 * ((size_t)n << (n - 1)) + 3 * ((size_t)8 << n) + 8 * (size_t)mp + CERT_PART * 8 + 8;
     }
+    size_t spare_bytes() const override {
+        size_t s = 0;
+        for (const DevBuf *d : {&qa, &qb, &outw, &mass, &dp, &obs, &p, &pfit_cur, &pfit_best, &res, &part, &count, &menu, &alt,
+                                &rows, &y, &bad})
+            s += d->bytes;
+        return s;
+    }
     // st: the stream whose work uses the arrays (the counters are zeroed on it)
     void ensure(int n_, ll mp_, cudaStream_t st, int slots = 1) {
         n = n_;
@@ -1516,6 +1523,13 @@ struct BatchWork : public BmWorkBase {
         pfit.ensure((size_t)K * (size_t)mp * 8);
         res.ensure((size_t)K * R_SLOTS * 8);
     }
+    bool give_back() override {
+        const bool any = draws.ptr || fits.ptr;
+        draws.release();
+        fits.release();
+        return any;
+    }
+    size_t spare_bytes() const override { return draws.bytes + fits.bytes; }
 };
 
 template <class T>
@@ -1536,9 +1550,11 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     size_t fr = 0, tot = 0;
     double frac = (bp && bp->mem_fraction > 0) ? bp->mem_fraction : 0.8;
     size_t per = batch_slot_bytes<T>(n, mp);
-    CertWork &CW = cert_work(c);
-    CW.ensure(n, mp, c.own);
+    CertWork &one = cert_work(c);
+    one.ensure(n, mp, c.own);
     RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
+    const ll want = std::min<ll>(B, bp && bp->slots > 0 ? bp->slots : 256);
+    if ((ll)((double)fr * frac / (double)per) < want && c.give_back()) RUMB_CUDA(cudaMemGetInfo(&fr, &tot));
     ll fit = (ll)((double)fr * frac / (double)per);
     int K = (bp && bp->slots > 0) ? bp->slots : (int)std::min<ll>(fit, 256);
     K = std::max(1, std::min(K, B));
@@ -1548,10 +1564,18 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     if (!slot) slot.reset(new BatchWork<T>());
     BatchWork<T> &W = *static_cast<BatchWork<T> *>(slot.get());
     W.ensure(n, mp, K);
+    // from here on this batch's own memory is not spare
+    struct InBatch {
+        bool &f;
+        explicit InBatch(bool &in) : f(in) { f = true; }
+        ~InBatch() { f = false; }
+    } in_batch(c.in_batch);
     // slots checked together: as many as a quarter gigabyte of certificate arrays holds, and within a
-    // tenth of what the states leave free (one at a time needs no more than a single solve's)
+    // tenth of what the states leave free (one at a time takes a single solve's)
     const size_t cert_budget = std::min<size_t>((size_t)256 << 20, (fr - std::min(fr, (size_t)K * per)) / 10);
     const int KC = (int)std::max<size_t>(1, std::min<size_t>((size_t)K, cert_budget / CertWork::slot_bytes(n, mp)));
+    if (KC > 1 && !c.batch_cert) c.batch_cert.reset(new CertWork());
+    CertWork &CW = KC > 1 ? *static_cast<CertWork *>(c.batch_cert.get()) : one;
     CW.ensure(n, mp, c.own, KC);
     // shared structure: observed positions, bits, per-menu masks, diagonal
     const DevProblem D = upload_problem(*pr, CW, st);

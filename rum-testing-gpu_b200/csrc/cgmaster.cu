@@ -124,6 +124,7 @@ CgMaster *cgmaster_create(Pricer *pr, const int32_t *alts, const double *p_obs, 
     std::unique_ptr<CgMaster> m(new CgMaster());
     m->pr = pr;
     m->c = &pricer_ctx(pr);
+    SpareGuard spare(m->c);
     m->n = n;
     m->M = M;
     m->W = (int)((M + 63) / 64);

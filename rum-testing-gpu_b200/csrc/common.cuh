@@ -48,6 +48,14 @@ inline thread_local long long g_launches = 0;
 void set_last_error(const std::string &msg);
 
 // ---------------------------------------------------------------- device buffers
+// What the calling thread's context holds beyond a call's needs and can give back when memory is short (set for
+// the length of a call; returns whether anything was freed).
+struct Spare {
+    virtual bool give_back() = 0;
+    virtual size_t bytes() const = 0;
+};
+inline thread_local Spare *g_spare = nullptr;
+
 // An owning device allocation. The library allocates through the context only (cudaMalloc on
 // the context's device); buffers are reused across solves of one shape.
 struct DevBuf {
@@ -80,7 +88,12 @@ struct DevBuf {
         if (b <= bytes && ptr) return;
         release();
         if (b == 0) return;
-        RUMB_CUDA(cudaMalloc(&ptr, b));
+        cudaError_t e = cudaMalloc(&ptr, b);
+        if (e == cudaErrorMemoryAllocation && g_spare && g_spare->give_back()) {
+            cudaGetLastError();
+            e = cudaMalloc(&ptr, b);
+        }
+        cuda_check(e, "cudaMalloc");
         bytes = b;
     }
     template <class T> T *as() const { return reinterpret_cast<T *>(ptr); }

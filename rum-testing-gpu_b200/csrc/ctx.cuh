@@ -13,9 +13,12 @@ namespace rumb {
 
 struct BmWorkBase {
     virtual ~BmWorkBase() {}
+    // what outlives a call only to save the next one's allocation: freed, counted
+    virtual bool give_back() { return false; }
+    virtual size_t spare_bytes() const { return 0; }
 };
 
-struct Ctx {
+struct Ctx : public Spare {
     int device = 0;
     cudaStream_t own = nullptr;       // the context's stream (work always runs here)
     cudaStream_t user = nullptr;      // optional caller stream, joined by events
@@ -27,6 +30,23 @@ struct Ctx {
     std::unique_ptr<BmWorkBase> bm64, bm32;     // BM-ADMM workspaces
     std::unique_ptr<BmWorkBase> batch64, batch32;  // batched-draw workspaces
     std::unique_ptr<BmWorkBase> cert;           // float64 certificate workspace
+    std::unique_ptr<BmWorkBase> batch_cert;     // a batch's, of several slots
+    bool in_batch = false;                      // its draws and slots are in use
+    // A batch's certificate slots and uploaded draws stay for the next batch, until another call needs their memory.
+    bool give_back() override {
+        if (in_batch) return false;
+        bool any = batch_cert != nullptr;
+        batch_cert.reset();
+        for (BmWorkBase *w : {batch64.get(), batch32.get()})
+            if (w && w->give_back()) any = true;
+        return any;
+    }
+    size_t bytes() const override {
+        size_t b = batch_cert ? batch_cert->spare_bytes() : 0;
+        for (const BmWorkBase *w : {batch64.get(), batch32.get()})
+            if (w) b += w->spare_bytes();
+        return b;
+    }
     std::unique_ptr<BmWorkBase> scratch;        // primitive calls' scratch
     // the captured iteration and check graphs of the last solve of each kind (bm.cu); after the workspaces
     // they launch on, so that they go first
@@ -64,6 +84,13 @@ struct Ctx {
         }
     }
     const int *layer_table(int n, std::vector<ll> &bounds);
+};
+
+// RAII: the context whose spare memory a call may take
+struct SpareGuard {
+    Spare *prev;
+    explicit SpareGuard(Spare *s) : prev(g_spare) { g_spare = s; }
+    ~SpareGuard() { g_spare = prev; }
 };
 
 // RAII: make ctx's device current for the duration of a call

@@ -319,6 +319,7 @@ void draws_rows(Draws *D, const int64_t *idx, ll count, int perturbed, double sc
     if (count == 0) return;
     for (ll i = 0; i < count; ++i)
         if (idx[i] < 0 || idx[i] >= D->B) fail(RUMB_E_INVAL, "draws: draw index out of range");
+    SpareGuard spare(D->c);
     cudaStream_t st = D->c->own;
     upload(D->idx, idx, (size_t)count, st);
     D->rows.ensure((size_t)count * D->M * sizeof(double));
@@ -330,6 +331,7 @@ void draws_rows(Draws *D, const int64_t *idx, ll count, int perturbed, double sc
 void draws_screen(Draws *D, const double *fit, double scale, double *dev, double *ub) {
     if (!dev && !ub) return;
     if (ub && !fit) fail(RUMB_E_INVAL, "draws: the screen's bound needs a fit");
+    SpareGuard spare(D->c);
     cudaStream_t st = D->c->own;
     if (fit) upload(D->fit, fit, (size_t)D->M, st);
     D->dev.ensure((size_t)D->B * sizeof(double));

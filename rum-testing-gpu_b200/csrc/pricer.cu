@@ -1636,6 +1636,7 @@ Pricer *pricer_create(Ctx &c, int n, ll mp, const uint64_t *menus, const int64_t
 
 void pricer_max64(Pricer *P, const double *scores_host, double *vmax) {
     Ctx &c = *P->c;
+    SpareGuard spare(&c);
     cudaStream_t st = c.own;
     const int n = P->n;
     ull cap = 0;
