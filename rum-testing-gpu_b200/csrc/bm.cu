@@ -975,14 +975,14 @@ static void key_add(std::vector<unsigned long long> &k, double v) {
 static void key_add(std::vector<unsigned long long> &k, const void *p) { k.push_back((unsigned long long)(uintptr_t)p); }
 template <class T>
 static std::vector<unsigned long long> graph_key(Ctx &c, const CertWork &CW, const IterPtrs<T> &I, const BmCoef &C, int n,
-                                                 int chunk, const void *snap) {
+                                                 int chunk, const void *obsbits, const void *snap) {
     std::vector<unsigned long long> k{(unsigned long long)n, (unsigned long long)CW.mp, (unsigned long long)chunk,
                                       (unsigned long long)C.lo_bits, (unsigned long long)C.prox_form,
                                       (unsigned long long)C.fuse, (unsigned long long)C.dr, (unsigned long long)I.slots};
     for (double v : {C.b1, C.b2, C.alpha, C.p}) key_add(k, v);
     for (const void *p : {(const void *)I.x2, (const void *)I.s, (const void *)I.y, (const void *)I.z, (const void *)I.x,
                           (const void *)I.Ax, (const void *)I.t1, (const void *)I.t2, (const void *)I.xhat,
-                          (const void *)I.diag, (const void *)I.menu_obs, (const void *)I.err, (const void *)I.active, snap})
+                          (const void *)I.diag, (const void *)I.menu_obs, (const void *)I.err, (const void *)I.active, obsbits, snap})
         key_add(k, p);
     for (const DevBuf *b : {&CW.qa, &CW.qb, &CW.outw, &CW.mass, &CW.dp, &CW.obs, &CW.p, &CW.pfit_cur, &CW.pfit_best, &CW.res,
                             &CW.part, &CW.count})
@@ -1120,7 +1120,7 @@ static bool run_leg(Ctx &c, CertWork &CW, BmWork<T> &W, const BmCoef &C, const r
     const bool graphs = par.use_graph != 0, overlap = graphs && par.overlap_check;
     if (graphs) {
         if (overlap) W.snap.ensure(((size_t)n << (n - 1)) * sizeof(T));
-        G.use(graph_key<T>(c, CW, iter_ptrs<T>(W), C, n, chunk, overlap ? W.snap.ptr : nullptr));
+        G.use(graph_key<T>(c, CW, iter_ptrs<T>(W), C, n, chunk, W.obsbits.ptr, overlap ? W.snap.ptr : nullptr));
         if (!g_iter.e) g_iter.capture(st, [&] { enqueue_iterations<T>(W, C, n, st, chunk); });
     }
     if (overlap) return run_leg_overlap<T>(c, CW, W, pr, par, L, t0, stall_exit, G, chunk, trace, user);
@@ -1690,7 +1690,7 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     auto t_setup = Clock::now();
     const int chunk = graph_chunk(par->check);
     SolveGraphs &G = solve_graphs(sizeof(T) == 8 ? c.batch_graphs64 : c.batch_graphs32);
-    G.use(graph_key<T>(c, CW, I, C, n, chunk, nullptr));
+    G.use(graph_key<T>(c, CW, I, C, n, chunk, W.obsbits.ptr, nullptr));
     Graph &g_iter = G.iter;
     if (!g_iter.e) g_iter.capture(st, [&] { enqueue_iterations_ptrs<T>(I, C, n, st, chunk); });
     std::vector<double> res((size_t)K * R_SLOTS);
