@@ -87,17 +87,18 @@ int rumb_ctx_destroy(rumb_ctx *ctx) {
     {
         rumb::DeviceGuard dg(ctx->c.device);
         cudaStreamSynchronize(ctx->c.own);
+        if (ctx->c.aux) cudaStreamSynchronize(ctx->c.aux);
+        // the graphs before the workspaces and streams they were captured on
+        for (auto *g : {&ctx->c.graphs64, &ctx->c.graphs32, &ctx->c.batch_graphs64, &ctx->c.batch_graphs32}) g->reset();
         ctx->c.bm64.reset();
         ctx->c.bm32.reset();
         ctx->c.batch64.reset();
         ctx->c.batch32.reset();
         ctx->c.cert.reset();
+        ctx->c.batch_cert.reset();
         ctx->c.scratch.reset();
         ctx->c.layers.clear();
-        if (ctx->c.aux) {
-            cudaStreamSynchronize(ctx->c.aux);
-            cudaStreamDestroy(ctx->c.aux);
-        }
+        if (ctx->c.aux) cudaStreamDestroy(ctx->c.aux);
         if (ctx->c.ev_snap) cudaEventDestroy(ctx->c.ev_snap);
         if (ctx->c.ev_done) cudaEventDestroy(ctx->c.ev_done);
         if (ctx->c.res_host) cudaFreeHost(ctx->c.res_host);

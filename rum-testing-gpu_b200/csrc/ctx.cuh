@@ -48,8 +48,8 @@ struct Ctx : public Spare {
         return b;
     }
     std::unique_ptr<BmWorkBase> scratch;        // primitive calls' scratch
-    // the captured iteration and check graphs of the last solve of each kind (bm.cu); after the workspaces
-    // they launch on, so that they go first
+    // the captured iteration and check graphs of the last solve of each kind (bm.cu; released before the
+    // workspaces they launch on)
     std::unique_ptr<BmWorkBase> graphs64, graphs32, batch_graphs64, batch_graphs32;
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;   // a call's device time (made on first use)
     // overlapped checks: a second stream and its two events; a check's pinned result words (made on first use)
