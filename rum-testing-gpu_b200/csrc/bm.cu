@@ -660,7 +660,7 @@ static DrArgs dr_args(const IterPtrs<double> &I, const BmCoef &C, int n) {
     P.kA = Co<double>{1.0, -1.0, 0.0, C.p};
     P.kAp = Co<double>{1.0, 0.0, -1.0, C.p};
     P.alpha = C.alpha; P.b = C.b2;
-    P.inv_c0 = 1.0 / C.b2; P.inv_c1 = 1.0 / (C.b2 + 2.0);
+    P.inv_c1 = 1.0 / (C.b2 + 2.0);
     P.bstride = P.tstride = I.bstride;
     P.active = I.active;
     return P;

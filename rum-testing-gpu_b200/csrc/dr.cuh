@@ -41,7 +41,7 @@ struct DrArgs {
     double *u_out, *t_out;      // the u and t slabs, written by the last iteration of a sequence
     const double *diag;         // eigen-space diagonal by popcount, with the unit forms' scales
     Co<double> kQ, kAQ, kA, kAp;   // Q (unit form), A Q / q00, A, A'
-    double alpha, b, inv_c0, inv_c1;   // b and 1 / b, 1 / (b + 2)
+    double alpha, b, inv_c1;    // b and 1 / (b + 2)
     ll bstride, tstride;        // batched draws: elements between draws' slabs and thresholds (grid.y)
     const int *active;
 };
