@@ -57,7 +57,6 @@ struct PricerArgs {
     float *mcur, *ecur;
     uint8_t *pred;             // nullptr when this layer keeps no predecessors
     unsigned int *layer_step;  // float bits, atomicMax (steps are >= 0)
-    unsigned int *bcnt;        // per quantization block: its finished CTAs (zero between launches), or nullptr
     // mask mode: the layer's nodes, values and predecessors indexed by the mask
     const int *nodes;
     float *vmask;
@@ -179,67 +178,6 @@ __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in
     return w_list(A.loffs, (const uint32_t *)A.lent, p, A.scores + lo);
 }
 
-// Quantizes block blk (1024 ranks) of a layer with `nt` threads (a multiple of 32): block min / max, step =
-// (max - min) / levels, q = rintf((v - min) / step). The values were written by this or other CTAs.
-__device__ __forceinline__ void quant_block(const PricerArgs &A, const float *vals, ull blk, int tid, int nt) {
-    __shared__ float smin[32], smax[32];
-    const ull r0 = blk * PB, end = r0 + PB < A.count ? r0 + PB : A.count;
-    float tmin = 3.0e38f, tmax = -3.0e38f;
-    for (ull r = r0 + tid; r < end; r += nt) {
-        const float v = __ldcg(vals + r);
-        tmin = fminf(tmin, v);
-        tmax = fmaxf(tmax, v);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
-        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-    }
-    if ((tid & 31) == 0) { smin[tid >> 5] = tmin; smax[tid >> 5] = tmax; }
-    __syncthreads();
-    float bmin = smin[0], bmax = smax[0];
-    for (int i = 1; i < nt / 32; ++i) { bmin = fminf(bmin, smin[i]); bmax = fmaxf(bmax, smax[i]); }
-    const float levels = A.mode == 2 ? 65535.0f : 16777215.0f;
-    const float step = __fdiv_rn(__fsub_rn(bmax, bmin), levels);
-    if (tid == 0) {
-        A.mcur[blk] = bmin;
-        A.ecur[blk] = step;
-        atomicMax(A.layer_step, __float_as_uint(step));
-    }
-    for (ull r = r0 + tid; r < end; r += nt) {
-        const float v = __ldcg(vals + r);
-        float q = (step > 0.0f) ? rintf(__fdiv_rn(__fsub_rn(v, bmin), step)) : 0.0f;
-        q = fminf(fmaxf(q, 0.0f), levels);
-        const unsigned int qi = (unsigned int)q;
-        if (A.mode == 2) {
-            A.vcur_h[r] = (uint16_t)qi;
-        } else {
-            A.vcur_h[r] = (uint16_t)(qi >> 8);
-            A.lcur[r] = (uint8_t)(qi & 255u);
-        }
-    }
-}
-
-// The end of a layer kernel's CTA that wrote ranks [r0, r0 + span) (span divides 1024): the last CTA of a
-// quantization block quantizes it, so that a layer is one launch (a launch of its own took 4 us of a layer's
-// 10 to 25 at n = 18). Every thread of the CTA calls it.
-__device__ __forceinline__ void finish_block(const PricerArgs &A, const float *vals, ull r0, int span) {
-    if (A.mode < 2 || !A.bcnt) return;
-    __shared__ int last;
-    __threadfence();
-    __syncthreads();
-    const ull blk = r0 / PB;
-    if (threadIdx.x == 0) {
-        const ull first = blk * PB, cnt = A.count - first < PB ? A.count - first : PB;
-        const unsigned parts = (unsigned)((cnt + span - 1) / span);
-        last = atomicAdd(A.bcnt + blk, 1u) + 1u == parts;
-        if (last) A.bcnt[blk] = 0u;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    quant_block(A, vals, blk, (int)threadIdx.x, (int)blockDim.x);
-}
-
 // One popcount layer k of the sweep.
 //
 // layer_eval_kernel: a CTA of 1024 threads covers PE_R = 128 consecutive ranks (32 ranks and 256
@@ -255,8 +193,10 @@ __device__ __forceinline__ void finish_block(const PricerArgs &A, const float *v
 //   stream: D is the colex unranking of r; the value of D \ {x} is read from the previous layer's
 //         storage at its colex rank; output: the float32 value (f32 mode, and the predecessor
 //         byte) or the value for stream_quant_kernel to quantize (u16 / u24).
-// Quantization blocks are 1024 ranks, as the number format asks (u16 / u24 modes): the last CTA of a block
-// quantizes it (finish_block), or stream_quant_kernel after the group sweep.
+// stream_quant_kernel: one CTA per quantization block of 1024 ranks, as the number format asks:
+// block min / max, step, rintf quantization of every value (u16 / u24 modes). A launch of its own and not the last
+// CTA of a block's: with the sums formed ahead its launch overlaps, and counting CTAs takes longer (n = 18, 0.5 % of
+// the menus, u24 262 us a call against 287, n = 14 131 / 155, n = 20, 0.3 % 829 / 885).
 constexpr int PE_R = 128, PE_G = 8;
 static_assert((PE_R / 32) * PE_G == 32 && (PE_G & (PE_G - 1)) == 0, "32 warps; PE_G a power of two");
 // Layers whose 128-rank CTAs would not give every SM two of them run 32 ranks per CTA (8 warps).
@@ -333,7 +273,6 @@ __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kern
             else vals[r] = b;
         }
     }
-    if (!MASK) finish_block(A, vals, (ull)blockIdx.x * PR, PR);
 }
 
 // The float64 max sweep (sweep_max64, the Frank-Wolfe bound's longest path when the float64 slab
@@ -462,7 +401,6 @@ __global__ void __launch_bounds__(1024) layer_wide_kernel(PricerArgs A, float *v
             else vals[r] = best;
         }
     }
-    if (!MASK) finish_block(A, vals, r, 1);
 }
 
 // Cover-list construction, once per pricer: thread per subset D (mask order, all layers in one
@@ -508,7 +446,36 @@ __global__ void stream_decode_kernel(PricerArgs A, ull count_prev, float *dec) {
 
 __global__ void __launch_bounds__(PB) stream_quant_kernel(PricerArgs A, const float *vals) {
     pdl_grid_sync();                                       // launched by launch_pdl
-    quant_block(A, vals, blockIdx.x, (int)threadIdx.x, PB);
+    __shared__ float smin[PB / 32], smax[PB / 32];
+    const ull r = (ull)blockIdx.x * PB + threadIdx.x;
+    const bool valid = r < A.count;
+    const float best = valid ? vals[r] : 0.0f;
+    float tmin = valid ? best : 3.0e38f, tmax = valid ? best : -3.0e38f;
+    for (int o = 16; o > 0; o >>= 1) {
+        tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+    }
+    if ((threadIdx.x & 31) == 0) { smin[threadIdx.x >> 5] = tmin; smax[threadIdx.x >> 5] = tmax; }
+    __syncthreads();
+    float bmin = smin[0], bmax = smax[0];
+    for (int i = 1; i < PB / 32; ++i) { bmin = fminf(bmin, smin[i]); bmax = fmaxf(bmax, smax[i]); }
+    const float levels = A.mode == 2 ? 65535.0f : 16777215.0f;
+    float step = __fdiv_rn(__fsub_rn(bmax, bmin), levels);
+    if (threadIdx.x == 0) {
+        A.mcur[blockIdx.x] = bmin;
+        A.ecur[blockIdx.x] = step;
+        atomicMax(A.layer_step, __float_as_uint(step));
+    }
+    if (!valid) return;
+    float q = (step > 0.0f) ? rintf(__fdiv_rn(__fsub_rn(best, bmin), step)) : 0.0f;
+    q = fminf(fmaxf(q, 0.0f), levels);
+    unsigned int qi = (unsigned int)q;
+    if (A.mode == 2) {
+        A.vcur_h[r] = (uint16_t)qi;
+    } else {
+        A.vcur_h[r] = (uint16_t)(qi >> 8);
+        A.lcur[r] = (uint8_t)(qi & 255u);
+    }
 }
 
 // Layer 0 (V[empty set] = 0: q 0, offset 0, step 0) and no steps yet, before a sweep of the stream storage.
@@ -1252,7 +1219,6 @@ struct Pricer {
     std::vector<std::unique_ptr<DevBuf>> pred;   // per layer >= k_pred
     DevBuf pred_ptrs;                       // device array of pred pointers (n+1)
     DevBuf layer_step;                      // n+1 uints (float bits)
-    DevBuf bcnt;                            // per quantization block: finished CTAs (quantized storage)
     DevBuf Vs, Ps;                          // sub-lattice / mask scratch
     DevBuf Ws;                              // sub-lattice sums w(x_j, D(s)): 2^k_pred * k_pred floats
     DevBuf vals;                            // a layer's float32 values before quantization
@@ -1606,10 +1572,6 @@ Pricer *pricer_create(Ctx &c, int n, ll mp, const uint64_t *menus, const int64_t
             P->m[i].ensure((size_t)nblk * 4);
             P->e[i].ensure((size_t)nblk * 4);
         }
-        if (mode >= 2) {
-            P->bcnt.ensure((size_t)nblk * 4);
-            RUMB_CUDA(cudaMemsetAsync(P->bcnt.ptr, 0, (size_t)nblk * 4, st));
-        }
         std::vector<uint8_t *> ptrs(n + 1, nullptr);
         P->pred.resize(n + 1);
         for (int k = P->k_pred; k <= n; ++k) {
@@ -1827,7 +1789,6 @@ static void run_sweep(Pricer *P, const float *scores) {
             A.ecur = P->e[cur].as<float>();
             A.pred = k >= P->k_pred ? P->pred[k]->as<uint8_t>() : nullptr;
             A.layer_step = P->layer_step.as<unsigned int>() + k;
-            if (!P->stream_group) A.bcnt = P->bcnt.as<unsigned int>();
             if (P->stream_group) {
                 const int hb = n - SG_LOW;
                 StreamGroupArgs G{};
@@ -1854,7 +1815,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             } else {
                 layer(A, false, P->vals.as<float>());
             }
-            if (A.mode != 1 && P->stream_group) {
+            if (A.mode != 1) {
                 launch_pdl(stream_quant_kernel, dim3((unsigned)((A.count + PB - 1) / PB)), dim3(PB), 0, st, A, P->vals.as<float>());
                 RUMB_LAUNCH("stream_quant_kernel");
             }
