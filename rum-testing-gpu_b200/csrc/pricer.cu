@@ -57,6 +57,7 @@ struct PricerArgs {
     float *mcur, *ecur;
     uint8_t *pred;             // nullptr when this layer keeps no predecessors
     unsigned int *layer_step;  // float bits, atomicMax (steps are >= 0)
+    unsigned int *bcnt;        // per quantization block: its finished CTAs (zero between launches), or nullptr
     // mask mode: the layer's nodes, values and predecessors indexed by the mask
     const int *nodes;
     float *vmask;
@@ -178,6 +179,65 @@ __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in
     return w_list(A.loffs, (const uint32_t *)A.lent, p, A.scores + lo);
 }
 
+// Quantizes block blk (1024 ranks) of a layer with `nt` threads (a multiple of 32): block min / max, step =
+// (max - min) / levels, q = rintf((v - min) / step). The values were written by this or other CTAs.
+__device__ __forceinline__ void quant_block(const PricerArgs &A, const float *vals, ull blk, int tid, int nt) {
+    __shared__ float smin[32], smax[32];
+    const ull r0 = blk * PB, end = r0 + PB < A.count ? r0 + PB : A.count;
+    float tmin = 3.0e38f, tmax = -3.0e38f;
+    for (ull r = r0 + tid; r < end; r += nt) {
+        const float v = __ldcg(vals + r);
+        tmin = fminf(tmin, v);
+        tmax = fmaxf(tmax, v);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+    }
+    if ((tid & 31) == 0) { smin[tid >> 5] = tmin; smax[tid >> 5] = tmax; }
+    __syncthreads();
+    float bmin = smin[0], bmax = smax[0];
+    for (int i = 1; i < nt / 32; ++i) { bmin = fminf(bmin, smin[i]); bmax = fmaxf(bmax, smax[i]); }
+    const float levels = A.mode == 2 ? 65535.0f : 16777215.0f;
+    const float step = __fdiv_rn(__fsub_rn(bmax, bmin), levels);
+    if (tid == 0) {
+        A.mcur[blk] = bmin;
+        A.ecur[blk] = step;
+        atomicMax(A.layer_step, __float_as_uint(step));
+    }
+    for (ull r = r0 + tid; r < end; r += nt) {
+        const float v = __ldcg(vals + r);
+        float q = (step > 0.0f) ? rintf(__fdiv_rn(__fsub_rn(v, bmin), step)) : 0.0f;
+        q = fminf(fmaxf(q, 0.0f), levels);
+        const unsigned int qi = (unsigned int)q;
+        if (A.mode == 2) {
+            A.vcur_h[r] = (uint16_t)qi;
+        } else {
+            A.vcur_h[r] = (uint16_t)(qi >> 8);
+            A.lcur[r] = (uint8_t)(qi & 255u);
+        }
+    }
+}
+
+// The end of a layer kernel's CTA that wrote ranks [r0, r0 + span) (span divides 1024): the last CTA of a
+// quantization block quantizes it. Every thread of the CTA calls it.
+__device__ __forceinline__ void finish_block(const PricerArgs &A, const float *vals, ull r0, int span) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    const ull blk = r0 / PB;
+    if (threadIdx.x == 0) {
+        const ull first = blk * PB, cnt = A.count - first < PB ? A.count - first : PB;
+        const unsigned parts = (unsigned)((cnt + span - 1) / span);
+        last = atomicAdd(A.bcnt + blk, 1u) + 1u == parts;
+        if (last) A.bcnt[blk] = 0u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    quant_block(A, vals, blk, (int)threadIdx.x, (int)blockDim.x);
+}
+
 // One popcount layer k of the sweep.
 //
 // layer_eval_kernel: a CTA of 1024 threads covers PE_R = 128 consecutive ranks (32 ranks and 256
@@ -194,9 +254,11 @@ __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in
 //         storage at its colex rank; output: the float32 value (f32 mode, and the predecessor
 //         byte) or the value for stream_quant_kernel to quantize (u16 / u24).
 // stream_quant_kernel: one CTA per quantization block of 1024 ranks, as the number format asks:
-// block min / max, step, rintf quantization of every value (u16 / u24 modes). A launch of its own and not the last
-// CTA of a block's: with the sums formed ahead its launch overlaps, and counting CTAs takes longer (n = 18, 0.5 % of
-// the menus, u24 262 us a call against 287, n = 14 131 / 155, n = 20, 0.3 % 829 / 885).
+// block min / max, step, rintf quantization of every value (u16 / u24 modes). With cover lists it is a launch of
+// its own: the sums formed ahead overlap it, and counting CTAs takes longer (n = 18, 0.5 % of the menus, u24 262 us a
+// call against 287, n = 14 131 / 155, n = 20, 0.3 % 829 / 885). Layers that scan rows run longer, and the CTAs of a launch
+// that waits for them would sit on their SMs: there the last CTA of a block quantizes it (FIN: finish_block; u16
+// without lists, n = 16, 1 % 272 us against 313, n = 18, 1 % 2,370 / 2,770, n = 20, 0.4 % 14,310 / 15,230).
 constexpr int PE_R = 128, PE_G = 8;
 static_assert((PE_R / 32) * PE_G == 32 && (PE_G & (PE_G - 1)) == 0, "32 warps; PE_G a power of two");
 // Layers whose 128-rank CTAs would not give every SM two of them run 32 ranks per CTA (8 warps).
@@ -209,7 +271,7 @@ constexpr int PE_R_SMALL = 32;
 // menus) 403 -> 300 us. Held to 32 registers, so that an SM's 2,048 threads are all there: where a thread
 // reads its lists or tests rows the loads' latency is hidden by warps alone (n = 20, 0.3 % of the menus, u24:
 // 1,005 us at 48 registers, 878 at 32; n = 22, pairs, row tests, u16: 2,841 and 2,265).
-template <bool MASK, int PR>
+template <bool MASK, int PR, bool FIN = false>
 __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kernel(PricerArgs A, float *vals) {
     pdl_launch_next();                                     // launched by launch_pdl
     static_assert(PR % 32 == 0 && (PR / 32) * PE_G <= 32, "at most 32 warps");
@@ -273,6 +335,7 @@ __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kern
             else vals[r] = b;
         }
     }
+    if (FIN) finish_block(A, vals, (ull)blockIdx.x * PR, PR);
 }
 
 // The float64 max sweep (sweep_max64, the Frank-Wolfe bound's longest path when the float64 slab
@@ -1219,6 +1282,7 @@ struct Pricer {
     std::vector<std::unique_ptr<DevBuf>> pred;   // per layer >= k_pred
     DevBuf pred_ptrs;                       // device array of pred pointers (n+1)
     DevBuf layer_step;                      // n+1 uints (float bits)
+    DevBuf bcnt;                            // per quantization block: finished CTAs (rows scanned, quantized storage)
     DevBuf Vs, Ps;                          // sub-lattice / mask scratch
     DevBuf Ws;                              // sub-lattice sums w(x_j, D(s)): 2^k_pred * k_pred floats
     DevBuf vals;                            // a layer's float32 values before quantization
@@ -1572,6 +1636,10 @@ Pricer *pricer_create(Ctx &c, int n, ll mp, const uint64_t *menus, const int64_t
             P->m[i].ensure((size_t)nblk * 4);
             P->e[i].ensure((size_t)nblk * 4);
         }
+        if (mode >= 2) {
+            P->bcnt.ensure((size_t)nblk * 4);
+            RUMB_CUDA(cudaMemsetAsync(P->bcnt.ptr, 0, (size_t)nblk * 4, st));
+        }
         std::vector<uint8_t *> ptrs(n + 1, nullptr);
         P->pred.resize(n + 1);
         for (int k = P->k_pred; k <= n; ++k) {
@@ -1695,10 +1763,12 @@ static void run_sweep(Pricer *P, const float *scores) {
                 constexpr int PR = PE_R_SMALL;
                 const unsigned grid = (unsigned)((A.count + PR - 1) / PR);
                 if (mask) launch_pdl(layer_eval_kernel<true, PR>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
+                else if (A.bcnt) launch_pdl(layer_eval_kernel<false, PR, true>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
                 else launch_pdl(layer_eval_kernel<false, PR>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
             } else {
                 const unsigned grid = (unsigned)((A.count + PE_R - 1) / PE_R);
                 if (mask) launch_pdl(layer_eval_kernel<true, PE_R>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
+                else if (A.bcnt) launch_pdl(layer_eval_kernel<false, PE_R, true>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
                 else launch_pdl(layer_eval_kernel<false, PE_R>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
             }
             RUMB_LAUNCH("layer_eval_kernel");
@@ -1789,6 +1859,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             A.ecur = P->e[cur].as<float>();
             A.pred = k >= P->k_pred ? P->pred[k]->as<uint8_t>() : nullptr;
             A.layer_step = P->layer_step.as<unsigned int>() + k;
+            if (A.mode >= 2 && P->wmode == W_SCAN && !P->stream_group) A.bcnt = P->bcnt.as<unsigned int>();
             if (P->stream_group) {
                 const int hb = n - SG_LOW;
                 StreamGroupArgs G{};
@@ -1815,7 +1886,7 @@ static void run_sweep(Pricer *P, const float *scores) {
             } else {
                 layer(A, false, P->vals.as<float>());
             }
-            if (A.mode != 1) {
+            if (A.mode != 1 && !A.bcnt) {
                 launch_pdl(stream_quant_kernel, dim3((unsigned)((A.count + PB - 1) / PB)), dim3(PB), 0, st, A, P->vals.as<float>());
                 RUMB_LAUNCH("stream_quant_kernel");
             }
