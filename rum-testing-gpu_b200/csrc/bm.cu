@@ -1565,11 +1565,11 @@ static int bm_solve_batch_t(Ctx &c, const rumb_bm_problem *pr, const rumb_bm_par
     BatchWork<T> &W = *static_cast<BatchWork<T> *>(slot.get());
     W.ensure(n, mp, K);
     // from here on this batch's own memory is not spare
-    struct InBatch {
-        bool &f;
-        explicit InBatch(bool &in) : f(in) { f = true; }
-        ~InBatch() { f = false; }
-    } in_batch(c.in_batch);
+    struct BatchNow {
+        const BmWorkBase *&now;
+        BatchNow(const BmWorkBase *&n, const BmWorkBase *w) : now(n) { now = w; }
+        ~BatchNow() { now = nullptr; }
+    } batch_now(c.batch_now, &W);
     // slots checked together: as many as a quarter gigabyte of certificate arrays holds, and within a
     // tenth of what the states leave free (one at a time takes a single solve's)
     const size_t cert_budget = std::min<size_t>((size_t)256 << 20, (fr - std::min(fr, (size_t)K * per)) / 10);

@@ -31,14 +31,13 @@ struct Ctx : public Spare {
     std::unique_ptr<BmWorkBase> batch64, batch32;  // batched-draw workspaces
     std::unique_ptr<BmWorkBase> cert;           // float64 certificate workspace
     std::unique_ptr<BmWorkBase> batch_cert;     // a batch's, of several slots
-    bool in_batch = false;                      // its draws and slots are in use
+    const BmWorkBase *batch_now = nullptr;      // the running batch's workspace: its draws and slots are in use
     // A batch's certificate slots and uploaded draws stay for the next batch, until another call needs their memory.
     bool give_back() override {
-        if (in_batch) return false;
-        bool any = batch_cert != nullptr;
-        batch_cert.reset();
+        bool any = !batch_now && batch_cert;
+        if (!batch_now) batch_cert.reset();
         for (BmWorkBase *w : {batch64.get(), batch32.get()})
-            if (w && w->give_back()) any = true;
+            if (w && w != batch_now && w->give_back()) any = true;
         return any;
     }
     size_t bytes() const override {

@@ -42,3 +42,25 @@ def test_solve_fits_beside_what_a_batch_left():
         assert (x["ub"], x["lb"], x["iters"]) == (y["ub"], y["lb"], y["iters"])
         np.testing.assert_array_equal(x["p_fit"], y["p_fit"])
     c.close()
+
+
+def test_batch_takes_what_the_other_state_dtype_left():
+    """A float32 batch leaves 60 MB of draws; with 40 MB free a float64 batch's own draws fit only in their place."""
+    c = _lib.Context(0)
+    m, a, p = mixture_instance(10, 1.0, K=8, N=100, seed=1)
+    B = (60 << 20) // (8 * p.size)
+    P = np.clip(p[None, :] + np.random.default_rng(1).normal(0, 0.02, (B, p.size)), 0.0, 1.0)
+    prob = c.bm_problem(10, m, a, p)
+    run = lambda dt: c.bm_solve_batch(prob, c.bm_params(O.beta_default(p.size), max_iter=50, abs_tol=0.0, rel_tol=None, dtype=dt),
+                                      P, below=np.full(B, 1e6), slots=1)[0]
+    run("float32")
+    c.bm_solve(prob, c.bm_params(O.beta_default(p.size), max_iter=50, abs_tol=0.0, rel_tol=None))
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = run("float64")
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    want = run("float64")
+    assert [(r["ub"], r["lb"], r["iters"]) for r in got] == [(r["ub"], r["lb"], r["iters"]) for r in want]
+    c.close()
