@@ -149,14 +149,20 @@ __device__ __forceinline__ float w_scan(const ull *menus, const float *scores, l
     return w;
 }
 
-// w(x, D) from pair p's cover list (sx = x's first score): eight entries and then their scores in flight
-// together, added in list order (the chain entry -> score -> add is what a layer of lists with tens of
-// entries waits for).
-template <class IT>
+// w(x, D) from pair p's cover list (sx = x's first score), added in list order. AHEAD (mask storage): eight entries
+// and then their scores in flight together; rank-indexed layers with lists take them one after the other, four
+// unrolled. Ahead / one after the other, us a call: even to n = 18; n = 20, 0.3 % of the menus, mask 460 / 475, u24
+// 828 / 792.
+template <bool AHEAD, class IT>
 __device__ __forceinline__ float w_list(const unsigned *offs, const IT *ent, ull p, const float *sx) {
     const unsigned b = __ldg(offs + p), e = __ldg(offs + p + 1);
-    constexpr int U = 8;
     float w = 0.0f;
+    if (!AHEAD) {
+#pragma unroll 4
+        for (unsigned i = b; i < e; ++i) w = __fadd_rn(w, __ldg(sx + __ldg(ent + i)));
+        return w;
+    }
+    constexpr int U = 8;
     for (unsigned i = b; i < e; i += U) {
         unsigned id[U];
         float sc[U];
@@ -171,12 +177,13 @@ __device__ __forceinline__ float w_list(const unsigned *offs, const IT *ent, ull
     return w;
 }
 
+template <bool AHEAD>
 __device__ __forceinline__ float w_of(const PricerArgs &A, int x, ull D, bool in, ull p) {
     const ll lo = A.offsets[x];
     if (A.wmode == W_SCAN) return w_scan(A.menus, A.scores, lo, A.offsets[x + 1], D, in);
     if (!in) return 0.0f;
-    if (A.wmode == W_LIST16) return w_list(A.loffs, (const uint16_t *)A.lent, p, A.scores + lo);
-    return w_list(A.loffs, (const uint32_t *)A.lent, p, A.scores + lo);
+    if (A.wmode == W_LIST16) return w_list<AHEAD>(A.loffs, (const uint16_t *)A.lent, p, A.scores + lo);
+    return w_list<AHEAD>(A.loffs, (const uint32_t *)A.lent, p, A.scores + lo);
 }
 
 // Quantizes block blk (1024 ranks) of a layer with `nt` threads (a multiple of 32): block min / max, step =
@@ -257,7 +264,7 @@ __device__ __forceinline__ void finish_block(const PricerArgs &A, const float *v
 // block min / max, step, rintf quantization of every value (u16 / u24 modes). With cover lists it is a launch of
 // its own: the sums formed ahead overlap it, and counting CTAs takes longer (n = 18, 0.5 % of the menus, u24 262 us a
 // call against 287, n = 14 131 / 155, n = 20, 0.3 % 829 / 885). Layers that scan rows run longer, and the CTAs of a launch
-// that waits for them would sit on their SMs: there the last CTA of a block quantizes it (FIN: finish_block; u16
+// that waits for them would sit on their SMs: there the last CTA of a block quantizes it (SCAN: finish_block; u16
 // without lists, n = 16, 1 % 272 us against 313, n = 18, 1 % 2,370 / 2,770, n = 20, 0.4 % 14,310 / 15,230).
 constexpr int PE_R = 128, PE_G = 8;
 static_assert((PE_R / 32) * PE_G == 32 && (PE_G & (PE_G - 1)) == 0, "32 warps; PE_G a power of two");
@@ -271,7 +278,7 @@ constexpr int PE_R_SMALL = 32;
 // menus) 403 -> 300 us. Held to 32 registers, so that an SM's 2,048 threads are all there: where a thread
 // reads its lists or tests rows the loads' latency is hidden by warps alone (n = 20, 0.3 % of the menus, u24:
 // 1,005 us at 48 registers, 878 at 32; n = 22, pairs, row tests, u16: 2,841 and 2,265).
-template <bool MASK, int PR, bool FIN = false>
+template <bool MASK, int PR, bool SCAN = false>
 __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kernel(PricerArgs A, float *vals) {
     pdl_launch_next();                                     // launched by launch_pdl
     static_assert(PR % 32 == 0 && (PR / 32) * PE_G <= 32, "at most 32 warps");
@@ -299,7 +306,7 @@ __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kern
         wsum[q] = 0.0f;
         if (x >= n) continue;                                // uniform per warp
         const bool in = valid && ((D >> x) & 1ULL);
-        wsum[q] = w_of(A, x, D, in, pbase + __popcll(D & ((1ULL << x) - 1ULL)));
+        wsum[q] = w_of<MASK || SCAN>(A, x, D, in, pbase + __popcll(D & ((1ULL << x) - 1ULL)));
     }
     pdl_wait();
     float best = 0.0f;
@@ -335,7 +342,7 @@ __global__ void __launch_bounds__(PR * PE_G, 2048 / (PR * PE_G)) layer_eval_kern
             else vals[r] = b;
         }
     }
-    if (FIN) finish_block(A, vals, (ull)blockIdx.x * PR, PR);
+    if (SCAN && A.bcnt) finish_block(A, vals, (ull)blockIdx.x * PR, PR);
 }
 
 // The float64 max sweep (sweep_max64, the Frank-Wolfe bound's longest path when the float64 slab
@@ -656,8 +663,8 @@ __global__ void backtrace_kernel(int n, int k_pred, const ull *binom, uint8_t *c
             const int c = __popcll(s);
             const ull p = layer_base[c] + colex_rank_dev(Dorig, sbin, n) * (ull)c +
                           __popcll(Dorig & ((1ULL << x) - 1ULL));
-            w = wmode == W_LIST16 ? w_list(loffs, (const uint16_t *)lent, p, scores + offsets[x])
-                                  : w_list(loffs, (const uint32_t *)lent, p, scores + offsets[x]);
+            w = wmode == W_LIST16 ? w_list<true>(loffs, (const uint16_t *)lent, p, scores + offsets[x])
+                                  : w_list<true>(loffs, (const uint32_t *)lent, p, scores + offsets[x]);
         }
         Ws[t] = w;
     }
@@ -1763,12 +1770,12 @@ static void run_sweep(Pricer *P, const float *scores) {
                 constexpr int PR = PE_R_SMALL;
                 const unsigned grid = (unsigned)((A.count + PR - 1) / PR);
                 if (mask) launch_pdl(layer_eval_kernel<true, PR>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
-                else if (A.bcnt) launch_pdl(layer_eval_kernel<false, PR, true>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
+                else if (P->wmode == W_SCAN) launch_pdl(layer_eval_kernel<false, PR, true>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
                 else launch_pdl(layer_eval_kernel<false, PR>, dim3(grid), dim3(PR * PE_G), 0, st, A, vals);
             } else {
                 const unsigned grid = (unsigned)((A.count + PE_R - 1) / PE_R);
                 if (mask) launch_pdl(layer_eval_kernel<true, PE_R>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
-                else if (A.bcnt) launch_pdl(layer_eval_kernel<false, PE_R, true>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
+                else if (P->wmode == W_SCAN) launch_pdl(layer_eval_kernel<false, PE_R, true>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
                 else launch_pdl(layer_eval_kernel<false, PE_R>, dim3(grid), dim3(PE_R * PE_G), 0, st, A, vals);
             }
             RUMB_LAUNCH("layer_eval_kernel");
