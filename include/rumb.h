@@ -84,6 +84,7 @@ RUMB_API int rumb_ctx_destroy(rumb_ctx *ctx);
  * own stream) */
 RUMB_API int rumb_ctx_set_stream(rumb_ctx *ctx, void *stream);
 RUMB_API int rumb_ctx_sync(rumb_ctx *ctx);
+/* free_bytes counts what a batch left with the context: a later call of it that needs the memory has it back */
 RUMB_API int rumb_mem_info(rumb_ctx *ctx, size_t *free_bytes, size_t *total_bytes);
 /* ask a running solve on ctx to stop at its next check (thread-safe) */
 RUMB_API int rumb_cancel(rumb_ctx *ctx);
